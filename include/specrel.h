@@ -520,17 +520,17 @@ typedef struct SrTuning {
     uint32_t leaf_coop;       /* 1: a warp tests the leaves of all its lanes together */
     uint32_t leaf_batch;      /* lanes on a leaf before the warp tests leaves: 1..32 */
     uint32_t home_pct;        /* share of the tiles (0..100) split into one band per SM, which the
-                                 warps on that SM take first; the rest go in frame order */
+                                 warps on that SM take first; the rest go in frame order (packet 0) */
     uint32_t stack_smem;      /* traversal-stack entries per thread kept in shared memory, 0..64
                                  (0: the whole stack in local memory); deeper entries go to local
                                  memory, so the visiting order does not depend on it */
     uint32_t top_levels;      /* levels of the wide tree staged in shared memory per block, 0..8
                                  (0: none); with stack_smem 0 or 12; the compact layout
                                  (sr_set_layout) stages none */
-    uint32_t packet;          /* 1 (the default): the warp walks its tile's primary rays as one
-                                 packet (one node sequence for its 32 rays, each lane with its
-                                 own closest hit), then its main-light shadow rays likewise; the
-                                 same hits as the per-ray order, equal-lambda ties included, as
+    uint32_t packet;          /* 1 (the default): a warp walks the 64 primary rays of a tile (the
+                                 shorter side of tile_w x tile_h doubled) as one packet, then its
+                                 main-light shadow rays likewise, over a layout of 32-wide nodes
+                                 built beside the others; the same hits as the per-ray order, equal-lambda ties included, as
                                  long as every hit lies beyond its leaf box's computed entry
                                  parameter (the records' 1e-4 box padding keeps a margin of
                                  1e-4 / |d| in ray parameter against its rounding); with

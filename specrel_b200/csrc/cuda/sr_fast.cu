@@ -2,9 +2,10 @@
 // launches (captured once into a CUDA graph and replayed):
 //
 //   k_camera_batch   FP64 observers (tetrad from rapidity in double, event rebased to the anchor)
-//   k_trace_lean     persistent traversal (the default schedule): warps take 32-ray tiles from a
-//                    global counter; each lane traces its pixel's primary ray (closest hit), then,
-//                    when the main light needs it, the shadow ray (any hit) in the same launch.
+//   k_fan_trace, k_fan_shadow   persistent traversal (the default): each warp walks the 64 rays of an
+//                    8x8-pixel tile as one packet (closest hits), then the main light's shadow rays.
+//   k_trace_lean     the same work ray by ray (SrTuning.packet = 0): warps take 32-ray tiles from a
+//                    global counter; each lane traces its pixel's primary ray, then its shadow ray.
 //   k_trace_batch    the same work under the other schedules of SrTuning (per-warp chunks of
 //                    tiles, partial refills, postponed or cooperative leaf tests).
 //   k_shade_batch    one thread per pixel: interpolation and shading, with the main light's
@@ -23,6 +24,7 @@
 #include "sr_fast.h"
 #include "sr_shade.cuh"
 #include "sr_traverse.cuh"
+#include "sr_fan.cuh"
 
 namespace srk {
 
@@ -135,6 +137,7 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
     if (e0 != cudaSuccess) return e0;
     fast_release(c);
     s.num_wide = 0;
+    s.fan_levels = 0;
     s.depth = depth;
     s.empty = n == 0;
     s.max_leaf = max_leaf;
@@ -156,7 +159,8 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
     s.root_ref = 0;  // internal root: wide node 0 (the top levels come first)
     size_t temp = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, temp, (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, st);
-    if ((e = s.scratch.ensure(3 * (size_t)n * 4 + 64 + temp + 512)) != cudaSuccess) return e;
+    const size_t fan_scratch = 6 * (size_t)n * 4 + sizeof(FanCounts);
+    if ((e = s.scratch.ensure(std::max(3 * (size_t)n * 4 + 64 + temp + 512, fan_scratch))) != cudaSuccess) return e;
     uint32_t* flags = s.scratch.as<uint32_t>();
     uint32_t* wid = flags + n;
     uint32_t* topid = wid + n;
@@ -196,9 +200,7 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
                                                  s.copies, s.refs.as<uint2>(), s.up.as<uint32_t>(),
                                                  s.leafpar.as<uint32_t>());
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    e = cudaStreamSynchronize(st);
-    s.scratch.ensure(0);
-    return e;
+    return fan_build(s, nodes, n, s.scratch.as<uint32_t>(), st);
 }
 
 SrTuning fast_default_tuning(const FastCtx& c) {
@@ -314,12 +316,11 @@ __device__ __forceinline__ bool ray_pixel(const TraceBatchArgs& a, uint32_t r, u
     uint32_t lt = t - __ldg(a.tile_pre + o);
     uint32_t x = (lt % od.tiles_x) * a.tile_w + l % a.tile_w;
     uint32_t y = (lt / od.tiles_x) * a.tile_h + l / a.tile_w;
-    if (x >= od.width || y >= od.height) return false;
     *obs = o;
     *px = x;
     *py = y;
     *p = od.pix_base + y * od.width + x;
-    return true;
+    return x < od.width && y < od.height;
 }
 
 // Shared memory of one warp for the cooperative leaf tests: the rays of the lanes at a leaf, and
@@ -629,6 +630,41 @@ __global__ void __launch_bounds__(512) k_trace_batch(TraceBatchArgs a) {
     }
 }
 
+// The main light's shadow query of a hit (compute_illumination's condition, renderer.rs:617-633).
+struct ShadowQuery {
+    float4 no, d, inv;
+    float t_min, t_max;
+    bool enters;  // the query's ray enters the scene's box
+};
+__device__ __forceinline__ bool casts_shadows(const SrGpuUniforms& U) {
+    return U.mode == 0u && U.shadow_mode != 0u && U.num_flashes == 0u;
+}
+// Whether the hit at `lambda` of the ray (-no, d) of observer `obs` casts one; fills `q`.
+__device__ __forceinline__ bool shadow_query(const TraceBatchArgs& a, uint32_t obs, uint32_t slot, float4 no, float4 d,
+                                             float lambda, ShadowQuery* q) {
+    const SrGpuUniforms& U = a.U[obs];
+    if (!casts_shadows(U)) return false;
+    const float4* at = a.attrs + 12u * slot;
+    const uint32_t mat = __float_as_uint(__ldg(at + 10).z);
+    if (__float_as_uint(__ldg(a.mats + 3u * mat + 2u).y) != 0u) return false;
+    const float4 ev = sub4(mul4(d, lambda), no);  // o + d * lambda
+    float4 tl;
+    float dist;
+    // The camera is read again here rather than kept in registers across the traversal.
+    light_ray(U, cam_of(a.cam, obs), ev, &tl, &dist);
+    if (!(fmaxf(rest_frame_cos(tl, __ldg(at + 8), __ldg(at + 9)), 0.0f) > 0.0f)) return false;
+    // Bvh4D::is_occluded(hit.event, to_light, 2e-3, dist - 2e-3) (renderer.rs:636-641).
+    q->no = neg4(ev);
+    q->d = tl;
+    q->inv = v4(safe_inv(tl.x), safe_inv(tl.y), safe_inv(tl.z), safe_inv(tl.w));
+    q->t_min = 2e-3f;
+    q->t_max = dist - 2e-3f;
+    float en, ex;
+    slab_interval(a.ws.root_min, a.ws.root_max, q->no, q->inv, q->t_min, q->t_max, &en, &ex);
+    q->enters = ex >= en;
+    return true;
+}
+
 // The default schedule (whole-tile refills, one tile per fetch, leaves tested per lane) in its lean
 // form: a warp takes the next 32-ray tile when all its lanes are done, and each lane runs its
 // primary query and then, when the main light needs it, its shadow query to the end, with no
@@ -670,11 +706,9 @@ __device__ __forceinline__ uint32_t next_tile(const TraceBatchArgs& a, uint32_t 
 // (SplitStack), the rest in local memory; SS == 0: all in local memory (LocalStack). OCT: the
 // scene has the 16 sign-octant box copies; otherwise the compact layout (one copy). TOP: the first
 // a.top_n wide nodes (the tree's top levels) are staged in shared memory after the stacks, their
-// (min, max) boxes then their references. PKT: each warp walks its tile's primary rays as one
-// packet (closest_packet; built with SS == 0, no staging and no counting).
-template <bool COUNT, int SS, bool OCT, bool TOP, bool PKT>
+// (min, max) boxes then their references.
+template <bool COUNT, int SS, bool OCT, bool TOP>
 __global__ void __launch_bounds__(512) k_trace_lean(const __grid_constant__ TraceBatchArgs a) {
-    static_assert(!PKT || (!COUNT && SS == 0 && !TOP), "the packet form is built alone");
     const uint32_t lane = threadIdx.x & 31u;
     Work wp{0, 0, 0}, wsh{0, 0, 0};
     uint2 lm[FAST_STACK];
@@ -702,12 +736,10 @@ __global__ void __launch_bounds__(512) k_trace_lean(const __grid_constant__ Trac
         const uint32_t base = tile << 5;
         uint32_t obs = 0, px = 0, py = 0, pix = 0;
         const bool valid = ray_pixel(a, base + lane, &obs, &px, &py, &pix);
-        if (!PKT && !valid) continue;  // the packet form keeps every lane in the warp's traversal
-        float4 o = v4(0.0f, 0.0f, 0.0f, 0.0f), d = v4(0.0f, 0.0f, 1.0f, 0.0f);
-        if (valid) {
-            float sx, sy;
-            camera_ray(a.U[obs], cam_of(a.cam, obs), px, py, &o, &d, &sx, &sy);
-        }
+        if (!valid) continue;
+        float4 o, d;
+        float sx, sy;
+        camera_ray(a.U[obs], cam_of(a.cam, obs), px, py, &o, &d, &sx, &sy);
         const float4 no = neg4(o);  // the traversal and the hit event use the negated origin only
         const float4 inv = v4(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z), safe_inv(d.w));
         float t_max = 180.0f;
@@ -716,60 +748,391 @@ __global__ void __launch_bounds__(512) k_trace_lean(const __grid_constant__ Trac
         if (!a.ws.empty) {
             float en, ex;
             slab_interval(a.ws.root_min, a.ws.root_max, no, inv, 1e-3f, t_max, &en, &ex);
-            const bool in = valid && ex >= en && en < t_max;  // else the ray misses the scene's box (bvh4d.rs:451)
-            if constexpr (PKT) {
-                if (__any_sync(0xFFFFFFFFu, in))
-                    slot = closest_packet<OCT>(a.ws, in, no, d, inv, 1e-3f, t_max, best, st, a.err);
-            } else if (in) {
-                slot = closest_lean<COUNT, OCT, TOP>(a.ws, a.ws.root_ref, no, d, inv, 1e-3f, t_max, best, st, a.err, wp,
-                                                     top);
-            }
+            if (ex >= en && en < t_max)  // else the ray misses the scene's box (bvh4d.rs:451)
+                slot = closest_lean<COUNT, OCT, TOP>(a.ws, a.ws.root_ref, no, d, inv, 1e-3f, t_max, best, st, a.err, wp, top);
         }
-        // The main light's shadow query of the pixel (compute_illumination's condition,
-        // renderer.rs:617-633): per lane, or, in the packet form, the warp's queries as one packet.
+        a.hits[pix] = make_float4(best.lambda, best.u, best.v, best.w);
+        a.slots[pix] = slot < 0 ? 0xFFFFFFFFu : (uint32_t)slot;
         uint8_t sh = 0;
-        bool shadow_in = false;
-        float4 sno = v4(0.0f, 0.0f, 0.0f, 0.0f), sd = v4(0.0f, 0.0f, 1.0f, 0.0f), sinv = v4(1.0f, 1.0f, 1.0f, 1.0f);
-        float s0 = 0.0f, s1 = 0.0f;
-        if (valid) {
-            const SrGpuUniforms& U = a.U[obs];
-            a.hits[pix] = make_float4(best.lambda, best.u, best.v, best.w);
-            a.slots[pix] = slot < 0 ? 0xFFFFFFFFu : (uint32_t)slot;
-            if (slot >= 0 && U.mode == 0u && U.shadow_mode != 0u && U.num_flashes == 0u) {
-                const float4* at = a.attrs + 12u * (uint32_t)slot;
-                const uint32_t mat = __float_as_uint(__ldg(at + 10).z);
-                if (__float_as_uint(__ldg(a.mats + 3u * mat + 2u).y) == 0u) {
-                    const float4 ev = sub4(mul4(d, best.lambda), no);  // o + d * lambda
-                    float4 tl;
-                    float dist;
-                    // The camera is read again here rather than kept in registers across the traversal.
-                    light_ray(U, cam_of(a.cam, obs), ev, &tl, &dist);
-                    if (fmaxf(rest_frame_cos(tl, __ldg(at + 8), __ldg(at + 9)), 0.0f) > 0.0f) {
-                        // Bvh4D::is_occluded(hit.event, to_light, 2e-3, dist - 2e-3) (renderer.rs:636-641).
-                        sh = 1;
-                        sno = neg4(ev);
-                        sd = tl;
-                        sinv = v4(safe_inv(tl.x), safe_inv(tl.y), safe_inv(tl.z), safe_inv(tl.w));
-                        s0 = 2e-3f;
-                        s1 = dist - 2e-3f;
-                        float en, ex;
-                        slab_interval(a.ws.root_min, a.ws.root_max, sno, sinv, s0, s1, &en, &ex);
-                        shadow_in = ex >= en;
-                    }
-                }
-            }
-        }
-        if constexpr (PKT) {
-            if (__any_sync(0xFFFFFFFFu, shadow_in) && any_packet<OCT>(a.ws, shadow_in, sno, sd, sinv, s0, s1, st, a.err))
+        ShadowQuery q;
+        if (slot >= 0 && shadow_query(a, obs, (uint32_t)slot, no, d, best.lambda, &q)) {
+            sh = 1;
+            if (q.enters && any_lean<COUNT, OCT, TOP>(a.ws, a.ws.root_ref, q.no, q.d, q.inv, q.t_min, q.t_max, st, a.err, wsh, top))
                 sh = 2;
-        } else if (shadow_in && any_lean<COUNT, OCT, TOP>(a.ws, a.ws.root_ref, sno, sd, sinv, s0, s1, st, a.err, wsh, top)) {
-            sh = 2;
         }
-        if (valid) a.shadow[pix] = sh;
+        a.shadow[pix] = sh;
     }
     if (COUNT) {
         add_work(a.work, wp);
         add_work(a.work + 3, wsh);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The packet form (SrTuning.packet): the walks of sr_fan.cuh in two persistent launches.
+//
+//   k_fan_trace    Every warp takes 8x8-pixel tiles (64 rays, two per lane) until there are none. A walk
+//                  of more than FAN_BUDGET steps is given up: its tile goes into a queue as eight
+//                  groups of 8 pixels, which the warps walk from the hits found, as they run out of tiles.
+//                  Pixels whose hits cast a shadow ray are listed, 32 (or a group) at a time.
+//   k_fan_shadow   The main light's shadow queries of the listed pixels. What a walk of more than
+//                  FAN_ANY_BUDGET steps leaves open goes into the queue, each query walked by a warp
+//                  alone.
+//
+// Rays that spread (small frames, and the views away from a fast observer's motion, which aberration
+// widens up to e^2|rapidity| times) make an interval that holds far more than they meet: one tile of a
+// 471x163 frame took 1.1 ms alone. Splitting such tiles in launches of their own left each launch
+// waiting for its last warps; from a queue the parts of a slow tile start while other tiles still run. One
+// launch for both kinds of rays was slower: its code misses the instruction cache (1.4 of 11 stall
+// cycles per instruction against 0.2 of 7).
+//
+// The queue: an entry is written at list[tail++]; a warp takes the ticket head++, and the entry of that
+// number is its next task, or there is none once all first tasks and every entry are finished. A warp
+// waits only for work that others are doing, which never waits for it, and for at most FAN_POLLS polls.
+// ---------------------------------------------------------------------------------------------
+constexpr uint32_t FAN_BUDGET = 400, FAN_ANY_BUDGET = 160;
+// Tests without a hit after which a tile's walk is given up. A walk given up costs more in parts (from
+// the root again, fewer rays per test), so a launch with much to do per warp gives up late (the 8-frame
+// launch of the 7.9M-tet workload: 2.10 ms of closest hits at 200 to 256, 2.40 at 128, 2.87 at 64), and a
+// small one, which its slowest tiles hold up, early (471x163 pixels seen at rapidity 1.7: 0.40 ms at 256,
+// 0.27 at 128).
+constexpr uint32_t FAN_WASTE = 256, FAN_WASTE_SMALL = 128, FAN_SMALL_TILES = 48u << 10;
+constexpr uint32_t FAN_UNLIMITED = 1u << 22;
+constexpr uint32_t FAN_GROUP_LOG = 3, FAN_PAIR_LOG = 1;  // log2 of a group's and a pair's pixels
+constexpr uint32_t FAN_POLLS = 1u << 21;
+// A task: tile * 64 + part + 1 (0: no entry yet). Parts of a tile in k_fan_trace's queue: its 8 groups of 8
+// pixels, then its 32 pairs; in the list of shadow rays: its two halves of 32 pixels, then its 8 groups, then
+// its 32 pairs; in k_fan_shadow's queue: its 64 pixels.
+constexpr uint32_t FAN_PARTS_LOG = 6, FAN_GROUPS = 8, FAN_HALVES = 2;
+constexpr uint32_t FAN_MAX_TILES = 1u << (31u - FAN_PARTS_LOG);
+constexpr uint32_t FAN_SHADOWS_PER_TILE = 32, FAN_QUEUED_PER_TILE = 64;
+// Counters, a line each for those that many warps change.
+enum { FAN_NEXT = 0, FAN_HEAD = 32, FAN_TAIL = 64, FAN_FINISHED = 96, FAN_FIRST_DONE = 97, FAN_COUNTERS = 128 };
+
+struct FanTasks {
+    uint32_t* count;    // FAN_COUNTERS words of this launch, zero at the start
+    uint32_t* list;     // the queue, zero at the start and again at the end
+    uint32_t* shadows;  // the pixels that cast shadow rays, as tasks
+    uint32_t* num_shadows;
+    uint32_t waste;     // FAN_WASTE or FAN_WASTE_SMALL
+};
+
+__device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// The observer of a tile and the tile's corner pixel.
+struct FanTile {
+    uint32_t obs, x, y;
+};
+__device__ __forceinline__ FanTile fan_tile(const TraceBatchArgs& a, uint32_t tile) {
+    FanTile t;
+    t.obs = find_obs(a.tile_pre, a.n, tile);
+    const uint32_t across = a.obs[t.obs].tiles_x, lt = tile - __ldg(a.tile_pre + t.obs), row = lt / across;
+    t.x = (lt - row * across) * a.tile_w;
+    t.y = row * a.tile_h;
+    return t;
+}
+__device__ __forceinline__ uint32_t warp_next(uint32_t* counter) {
+    uint32_t t = 0;
+    if ((threadIdx.x & 31u) == 0) t = atomicAdd(counter, 1u);
+    return __shfl_sync(FULL_WARP, t, 0);
+}
+// Puts a task (tile, part) for each lane that has one at the end of `list`.
+__device__ __forceinline__ void fan_list(uint32_t* list, uint32_t* tail, uint32_t tile, uint32_t part, bool has) {
+    const uint32_t lane = threadIdx.x & 31u, which = __ballot_sync(FULL_WARP, has);
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(tail, (uint32_t)__popc(which));
+    at = __shfl_sync(FULL_WARP, at, 0) + (uint32_t)__popc(which & ((1u << lane) - 1u));
+    if (has) *(volatile uint32_t*)(list + at) = (tile << FAN_PARTS_LOG) + part + 1u;
+}
+// The same into the queue, after this warp's writes.
+__device__ __forceinline__ void fan_push(const FanTasks& q, uint32_t tile, uint32_t part, bool has) {
+    __threadfence();
+    __syncwarp();
+    fan_list(q.list, q.count + FAN_TAIL, tile, part, has);
+}
+// A warp's first tasks are done: `mine` of them.
+__device__ __forceinline__ void fan_first_done(const FanTasks& q, uint32_t mine) {
+    __threadfence();
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0 && mine) atomicAdd(q.count + FAN_FIRST_DONE, mine);
+}
+__device__ __forceinline__ void fan_finished(const FanTasks& q) {
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0) {
+        __threadfence();
+        atomicAdd(q.count + FAN_FINISHED, 1u);
+    }
+}
+// The next task of the queue, or 0 when all work is done (`first`: the number of first tasks).
+__device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, uint32_t* err) {
+    uint32_t entry = 0;
+    if ((threadIdx.x & 31u) == 0) {
+        const uint32_t ticket = atomicAdd(q.count + FAN_HEAD, 1u);
+        for (uint32_t polls = 0;; ++polls) {
+            if (load_acquire(q.count + FAN_TAIL) > ticket) {
+                entry = load_acquire(q.list + ticket);
+                if (entry) {
+                    q.list[ticket] = 0u;
+                    break;
+                }
+            } else {
+                // Finished entries are counted after what they queued: with every first task done and as
+                // many entries finished as queued, nothing more will be.
+                if (load_acquire(q.count + FAN_FIRST_DONE) == first) {
+                    const uint32_t finished = load_acquire(q.count + FAN_FINISHED);
+                    const uint32_t tail = load_acquire(q.count + FAN_TAIL);
+                    if (finished == tail && tail <= ticket) break;
+                }
+                __nanosleep(1000);
+            }
+            if (polls > FAN_POLLS) {
+                atomicOr(err, ERR_BAD_INDEX);
+                break;
+            }
+        }
+    }
+    return __shfl_sync(FULL_WARP, entry, 0);
+}
+
+// The ray of a pixel, and what is written of its hit: out of line, one copy for the rays of a lane (two in
+// line make the tile's straight code too long for the instruction cache).
+struct FanRay {
+    float4 d, inv;
+};
+static __device__ __noinline__ FanRay fan_ray(const SrGpuUniforms* U, const float4* cam, uint32_t obs, uint32_t px, uint32_t py) {
+    float4 o;
+    FanRay r;
+    float sx, sy;
+    camera_ray(U[obs], cam_of(cam, obs), px, py, &o, &r.d, &sx, &sy);
+    r.inv = v4(safe_inv(r.d.x), safe_inv(r.d.y), safe_inv(r.d.z), safe_inv(r.d.w));
+    return r;
+}
+// The negated origin of an observer's rays: camera_ray's, the same for every pixel.
+__device__ __forceinline__ float4 fan_origin(const SrGpuUniforms& U, const Cam& c) {
+    float4 o = c.pos;
+    if (U.slice_mode == 2u) o = sub4(o, mul4(c.e0, U.frontier_view_offset));
+    if (U.slice_mode == 3u) o = add4(o, mul4(c.e0, U.prophecy_delta));
+    return neg4(o);
+}
+// Returns whether the hit casts a shadow ray.
+static __device__ __noinline__ bool fan_write(const TraceBatchArgs& a, uint32_t obs, uint32_t pix, uint32_t slot, float lambda,
+                                              float4 d, float4 no) {
+    // The barycentrics of the hit, as the test computed them (kept there, they would take registers
+    // through the walk).
+    const float4* g = a.ws.geoms + 5u * slot;
+    const float4 v0 = __ldg(g);
+    const float4 ev = sub4(mul4(d, lambda), no);
+    const float2 q01 = add2(f2(ev.x, ev.y), f2(-v0.x, -v0.y)), q23 = add2(f2(ev.z, ev.w), f2(-v0.z, -v0.w));
+    const float4 q = make_float4(q01.x, q01.y, q23.x, q23.y);
+    a.hits[pix] = make_float4(lambda, edot_p(__ldg(g + 2), q), edot_p(__ldg(g + 3), q), edot_p(__ldg(g + 4), q));
+    a.shadow[pix] = 0;
+    ShadowQuery sq;
+    return shadow_query(a, obs, slot, no, d, lambda, &sq);
+}
+
+// The closest hits of a rectangle of 2^(w_log + h_log) pixels of observer `obs` with corner (x0, y0);
+// `resume`: the hits in memory are kept as bounds. Returns false when the walk was given up; `casts`: bit
+// r set when one of the first (0) or second half (1) of the pixels has a hit that casts a shadow ray.
+template <bool OCT>
+__device__ __forceinline__ bool fan_pixels(const TraceBatchArgs& a, uint32_t obs, uint32_t x0, uint32_t y0, uint32_t w_log,
+                                           uint32_t h_log, bool resume, uint32_t budget, uint32_t waste, FanQueue& f, uint2* st,
+                                           uint32_t* casts) {
+    const uint32_t lane = threadIdx.x & 31u, half = 1u << (w_log + h_log - 1u);
+    const ObsDev& od = a.obs[obs];
+    float4 d[FAN_RAYS];
+    float t_max[FAN_RAYS];
+    int slot[FAN_RAYS];
+#pragma unroll
+    for (int r = 0; r < FAN_RAYS; ++r) {
+        d[r] = v4(0.0f, 0.0f, 0.0f, 0.0f);
+        t_max[r] = 0.0f;
+        slot[r] = -1;
+    }
+    {
+        const Cam cam = cam_of(a.cam, obs);
+        fan_bounds(a.U[obs], cam, fan_origin(a.U[obs], cam), x0, y0, w_log, h_log, f.rays);
+    }
+    auto rays = [&]() {
+        const float4 no = f.rays.no;
+#pragma unroll
+        for (int r = 0; r < FAN_RAYS; ++r) {
+            const uint32_t i = (uint32_t)r * half + lane;
+            const uint32_t px = x0 + (i & ((1u << w_log) - 1u)), py = y0 + (i >> w_log);
+            const FanRay ray = fan_ray(a.U, a.cam, obs, px, py);
+            d[r] = ray.d;
+            float en, ex;
+            slab_interval(a.ws.root_min, a.ws.root_max, no, ray.inv, 1e-3f, 180.0f, &en, &ex);
+            // Pixels outside the frame take no part, nor do rays that miss the scene's box (bvh4d.rs:451).
+            const bool in = lane < half && px < od.width && py < od.height && ex >= en && en < 180.0f;
+            t_max[r] = in ? 180.0f : 0.0f;
+            if (resume && in) {
+                const uint32_t pix = od.pix_base + py * od.width + px;
+                slot[r] = (int)__ldcg(a.slots + pix);
+                if (slot[r] >= 0) t_max[r] = __ldcg(&a.hits[pix].x);
+            }
+        }
+    };
+    bool done = true, ready = false;
+    if (!a.ws.empty) {
+        if (resume) {
+            rays();
+            ready = true;
+        }
+        done = closest_fan<OCT>(a.ws, rays, ready, d, 1e-3f, budget, waste, slot, t_max, f, st, a.err);
+    }
+    *casts = 0;
+#pragma unroll
+    for (int r = 0; r < FAN_RAYS; ++r) {
+        const uint32_t i = (uint32_t)r * half + lane;
+        const uint32_t px = x0 + (i & ((1u << w_log) - 1u)), py = y0 + (i >> w_log);
+        bool query = false;
+        if (lane < half && px < od.width && py < od.height) {
+            const uint32_t pix = od.pix_base + py * od.width + px;
+            a.slots[pix] = (uint32_t)slot[r];
+            if (slot[r] >= 0) query = fan_write(a, obs, pix, (uint32_t)slot[r], t_max[r], d[r], f.rays.no) && done;
+        }
+        if (__any_sync(FULL_WARP, query)) *casts |= 1u << r;
+    }
+    return done;
+}
+
+// The shadow query of a pixel with a hit; false: it casts none.
+__device__ __forceinline__ bool fan_query(const TraceBatchArgs& a, uint32_t obs, uint32_t px, uint32_t py, uint32_t pix,
+                                          ShadowQuery* q) {
+    const uint32_t slot = __ldcg(a.slots + pix);
+    if (slot == 0xFFFFFFFFu) return false;
+    float4 o, d;
+    float sx, sy;
+    camera_ray(a.U[obs], cam_of(a.cam, obs), px, py, &o, &d, &sx, &sy);
+    return shadow_query(a, obs, slot, neg4(o), d, __ldcg(&a.hits[pix].x), q);
+}
+
+// The parts of 2^size_log pixels of a tile: the longer side halved (the height on a tie).
+struct FanParts {
+    uint32_t w_log, h_log, across;  // log2 of a part's size and of the parts in a row
+};
+__device__ __forceinline__ FanParts fan_parts(uint32_t tw_log, uint32_t th_log, uint32_t size_log) {
+    FanParts g{tw_log, th_log, 0u};
+    while (g.w_log + g.h_log > size_log) {
+        if (g.w_log > g.h_log) --g.w_log;
+        else --g.h_log;
+    }
+    g.across = tw_log - g.w_log;
+    return g;
+}
+__device__ __forceinline__ uint32_t part_x(const FanParts& g, uint32_t part) { return (part & ((1u << g.across) - 1u)) << g.w_log; }
+__device__ __forceinline__ uint32_t part_y(const FanParts& g, uint32_t part) { return (part >> g.across) << g.h_log; }
+
+// 96 registers (it takes 114 unbounded, without a spill either way) leave room for 20 warps per SM instead of
+// 16: the 8-frame launch's closest hits 2.10 ms against 2.29. At 80 it spills and takes 2.37.
+template <bool OCT>
+__global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchArgs a, const FanTasks q) {
+    extern __shared__ FanQueue sm_queue[];
+    FanQueue& sm = sm_queue[threadIdx.x >> 5];
+    uint2 st[FAN_LEVELS];
+    const uint32_t tiles = a.total_rays >> 5, tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t mine = 0;
+    bool whole = true;  // whole tiles first, then the queue
+    for (;;) {
+        uint32_t tile, part = 0;
+        if (whole) {
+            tile = warp_next(q.count + FAN_NEXT);
+            if (tile >= tiles) {
+                fan_first_done(q, mine);
+                whole = false;
+            }
+        }
+        if (!whole) {
+            const uint32_t task = fan_take(q, tiles, a.err);
+            if (!task) break;
+            tile = (task - 1u) >> FAN_PARTS_LOG;
+            part = (task - 1u) & ((1u << FAN_PARTS_LOG) - 1u);
+        }
+        const FanTile t = fan_tile(a, tile);
+        const bool pair = part >= FAN_GROUPS;
+        if (pair) part -= FAN_GROUPS;
+        const FanParts g = fan_parts(tw_log, th_log, whole ? tw_log + th_log : (pair ? FAN_PAIR_LOG : FAN_GROUP_LOG));
+        const uint32_t x0 = part_x(g, part), y0 = part_y(g, part);  // in the tile
+        uint32_t casts;
+        const bool done = fan_pixels<OCT>(a, t.obs, t.x + x0, t.y + y0, g.w_log, g.h_log, !whole, pair ? FAN_UNLIMITED : FAN_BUDGET,
+                                          pair ? FAN_UNLIMITED : q.waste, sm, st, &casts);
+        if (!done) {
+            // A tile into groups; a group into its pairs, numbered over the tile.
+            const FanParts p = fan_parts(tw_log, th_log, FAN_PAIR_LOG);
+            // Pairs lie along rows (the last halving is of the height), as a group's pixels 2 k and 2 k + 1 do.
+            const uint32_t px = x0 + ((2u * lane) & ((1u << g.w_log) - 1u)), py = y0 + ((2u * lane) >> g.w_log);
+            if (pair) {
+                if (lane == 0) atomicOr(a.err, ERR_TRAVERSAL_LIMIT);
+            } else if (whole) {
+                fan_push(q, tile, lane, lane < FAN_GROUPS);
+            } else {
+                fan_push(q, tile, FAN_GROUPS + ((py >> p.h_log) << p.across) + (px >> p.w_log), lane < (1u << (FAN_GROUP_LOG - FAN_PAIR_LOG)));
+            }
+        } else if (casts) {
+            fan_list(q.shadows, q.num_shadows, tile, whole ? lane : FAN_HALVES + part + (pair ? FAN_GROUPS : 0u),
+                     lane < 2u && (whole ? (casts >> lane) & 1u : lane == 0u));
+        }
+        if (whole) ++mine;
+        else fan_finished(q);
+    }
+}
+
+__global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ TraceBatchArgs a, const FanTasks q) {
+    extern __shared__ FanShadows sm_shadows[];
+    FanShadows& sm = sm_shadows[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    uint2 st[FAN_LEVELS];
+    const uint32_t tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
+    const uint32_t tasks = *q.num_shadows, part_mask = (1u << FAN_PARTS_LOG) - 1u;
+    uint32_t mine = 0;
+    for (;;) {
+        const uint32_t next = warp_next(q.count + FAN_NEXT);
+        if (next >= tasks) break;
+        const uint32_t task = q.shadows[next] - 1u, tile = task >> FAN_PARTS_LOG, part = task & part_mask;
+        const bool half = part < FAN_HALVES, pair = part >= FAN_HALVES + FAN_GROUPS;
+        const FanParts g = fan_parts(tw_log, th_log, half ? tw_log + th_log : (pair ? FAN_PAIR_LOG : FAN_GROUP_LOG));
+        const uint32_t k = half ? 0u : part - FAN_HALVES - (pair ? FAN_GROUPS : 0u);
+        const FanTile t = fan_tile(a, tile);
+        const uint32_t i = half ? 32u * part + lane : lane, n = half ? 64u : 1u << (g.w_log + g.h_log);
+        const uint32_t x = part_x(g, k) + (i & ((1u << g.w_log) - 1u)), y = part_y(g, k) + (i >> g.w_log);  // in the tile
+        const ObsDev& od = a.obs[t.obs];
+        const uint32_t px = t.x + x, py = t.y + y, pix = od.pix_base + py * od.width + px;
+        ShadowQuery s;
+        s.no = v4(0.0f, 0.0f, 0.0f, 0.0f);
+        s.d = v4(0.0f, 0.0f, 1.0f, 0.0f);
+        s.t_max = 0.0f;
+        s.enters = false;
+        const bool query = i < n && px < od.width && py < od.height &&
+                           fan_query(a, t.obs, px, py, pix, &s);
+        const bool enters = query && s.enters;
+        bool hit = false, done = true;
+        if (__any_sync(FULL_WARP, enters))
+            done = any_fan(a.ws, enters, s.no, s.d, 2.0f * (float)x / (float)(a.tile_w - 1u) - 1.0f,
+                           2.0f * (float)y / (float)(a.tile_h - 1u) - 1.0f, 2e-3f, s.t_max, FAN_ANY_BUDGET, hit, sm, st);
+        const bool pending = !done && enters && !hit;
+        if (query) a.shadow[pix] = hit ? 2 : 1;
+        if (__any_sync(FULL_WARP, pending)) fan_push(q, tile, (y << tw_log) + x, pending);
+        ++mine;
+    }
+    fan_first_done(q, mine);
+    for (;;) {
+        const uint32_t task = fan_take(q, tasks, a.err);
+        if (!task) break;
+        const uint32_t i = (task - 1u) & part_mask;
+        const FanTile t = fan_tile(a, (task - 1u) >> FAN_PARTS_LOG);
+        const ObsDev& od = a.obs[t.obs];
+        const uint32_t px = t.x + (i & ((1u << tw_log) - 1u)), py = t.y + (i >> tw_log), pix = od.pix_base + py * od.width + px;
+        ShadowQuery s;
+        if (fan_query(a, t.obs, px, py, pix, &s)) {  // the same for every lane
+            const bool hit = any_fan_one(a.ws, s.no, s.d, s.t_min, s.t_max, st, a.err);
+            if (lane == 0) a.shadow[pix] = hit ? 2 : 1;
+        }
+        fan_finished(q);
     }
 }
 
@@ -788,7 +1151,7 @@ bool lean_stack_supported(uint32_t s) {
 template <bool COUNT, int SS, bool OCT, bool TOP>
 static cudaError_t lean_attr(int max_smem) {
     return SS > 0 || TOP
-               ? cudaFuncSetAttribute(k_trace_lean<COUNT, SS, OCT, TOP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+               ? cudaFuncSetAttribute(k_trace_lean<COUNT, SS, OCT, TOP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       max_smem)
                : cudaSuccess;
 }
@@ -820,29 +1183,22 @@ static void launch_lean_ss(bool count, bool oct, bool top, uint32_t blocks, uint
                            const TraceBatchArgs& ta) {
     if constexpr (SS == 0 || SS == 12) {
         if (top && oct) {
-            if (count) k_trace_lean<true, SS, true, true, false><<<blocks, threads, smem, st>>>(ta);
-            else k_trace_lean<false, SS, true, true, false><<<blocks, threads, smem, st>>>(ta);
+            if (count) k_trace_lean<true, SS, true, true><<<blocks, threads, smem, st>>>(ta);
+            else k_trace_lean<false, SS, true, true><<<blocks, threads, smem, st>>>(ta);
             return;
         }
     }
     if (oct) {
-        if (count) k_trace_lean<true, SS, true, false, false><<<blocks, threads, smem, st>>>(ta);
-        else k_trace_lean<false, SS, true, false, false><<<blocks, threads, smem, st>>>(ta);
+        if (count) k_trace_lean<true, SS, true, false><<<blocks, threads, smem, st>>>(ta);
+        else k_trace_lean<false, SS, true, false><<<blocks, threads, smem, st>>>(ta);
     } else {
-        if (count) k_trace_lean<true, SS, false, false, false><<<blocks, threads, smem, st>>>(ta);
-        else k_trace_lean<false, SS, false, false, false><<<blocks, threads, smem, st>>>(ta);
+        if (count) k_trace_lean<true, SS, false, false><<<blocks, threads, smem, st>>>(ta);
+        else k_trace_lean<false, SS, false, false><<<blocks, threads, smem, st>>>(ta);
     }
 }
 
-// packet: the warp-packet traversal of primary rays (counting runs always take the per-lane order,
-// whose work counts are the reference traversal's).
-static void launch_lean(uint32_t ss, bool count, bool oct, bool top, bool packet, uint32_t blocks, uint32_t threads,
-                        size_t smem, cudaStream_t st, const TraceBatchArgs& ta) {
-    if (packet && !count) {
-        if (oct) k_trace_lean<false, 0, true, false, true><<<blocks, threads, smem, st>>>(ta);
-        else k_trace_lean<false, 0, false, false, true><<<blocks, threads, smem, st>>>(ta);
-        return;
-    }
+static void launch_lean(uint32_t ss, bool count, bool oct, bool top, uint32_t blocks, uint32_t threads, size_t smem,
+                        cudaStream_t st, const TraceBatchArgs& ta) {
 #define SR_ONE(S)                                                             \
     if (ss == (S)) {                                                          \
         launch_lean_ss<(S)>(count, oct, top, blocks, threads, smem, st, ta);  \
@@ -957,7 +1313,7 @@ struct Shape {
     std::vector<uint32_t> pre;  // (SR_BLOOM_LEVELS + 3) rows of n + 1: tiles, levels 0..6, star tiles
 };
 
-Shape make_shape(const BatchRequest& r, const SrTuning& t) {
+Shape make_shape(const BatchRequest& r, uint32_t tile_w, uint32_t tile_h) {
     Shape s;
     s.n = r.n;
     s.obs.resize(r.n);
@@ -970,7 +1326,7 @@ Shape make_shape(const BatchRequest& r, const SrTuning& t) {
         std::memset(&o, 0, sizeof(o));
         o.width = r.u[i].size[0];
         o.height = r.u[i].size[1];
-        o.tiles_x = (o.width + t.tile_w - 1) / t.tile_w;
+        o.tiles_x = (o.width + tile_w - 1) / tile_w;
         o.tile_base = tiles;
         o.pix_base = px;
         o.pyr_base = pyr;
@@ -986,7 +1342,7 @@ Shape make_shape(const BatchRequest& r, const SrTuning& t) {
             uint32_t* row = &s.pre[(size_t)(1 + k) * stride];
             row[i + 1] = row[i] + p.w[k] * p.h[k];
         }
-        tiles += o.tiles_x * ((o.height + t.tile_h - 1) / t.tile_h);
+        tiles += o.tiles_x * ((o.height + tile_h - 1) / tile_h);
         px += o.width * o.height;
         pyr += p.off[SR_BLOOM_LEVELS + 1];
     }
@@ -1008,7 +1364,31 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                               cudaStream_t st) {
     if (r.n == 0) return cudaSuccess;
     c.adj_valid = false;  // the batch buffers the gradient's outcomes live in are about to change
-    Shape sh = make_shape(r, t);
+    // The packet walk; counting runs take the per-lane order, whose work counts are the reference's.
+    bool packet = t.packet != 0 && !r.count_work && (s.empty || s.fan_levels != 0);
+    Shape sh;
+    uint32_t tile_w = t.tile_w, tile_h = t.tile_h;
+    if (packet) {  // 64-pixel tiles: the shorter side doubled
+        (tile_w < tile_h ? tile_w : tile_h) *= 2;
+        sh = make_shape(r, tile_w, tile_h);
+        const size_t old = c.fan_list.bytes, old_shadows = c.fan_shadows.bytes;
+        // Without room for the queue the rays walk alone. The queue's own buffer: its entries are zero
+        // between launches, whatever the next one's size, the list's are not.
+        packet = sh.total_tiles < FAN_MAX_TILES &&
+                 c.fan_list.ensure((size_t)sh.total_tiles * FAN_QUEUED_PER_TILE * 4) == cudaSuccess &&
+                 c.fan_shadows.ensure((size_t)sh.total_tiles * FAN_SHADOWS_PER_TILE * 4) == cudaSuccess;
+        if (c.fan_list.bytes != old || c.fan_shadows.bytes != old_shadows) fast_release(c);
+        if (c.fan_list.bytes != old && c.fan_list.p) {
+            cudaError_t z = cudaMemsetAsync(c.fan_list.p, 0, c.fan_list.bytes, st);
+            if (z != cudaSuccess) return z;
+        }
+        if (!packet) cudaGetLastError();
+    }
+    if (!packet) {
+        tile_w = t.tile_w;
+        tile_h = t.tile_h;
+        sh = make_shape(r, tile_w, tile_h);
+    }
     const uint32_t n = r.n, stride = n + 1;
     if ((uint64_t)sh.total_tiles * 32 >= (1ull << 32)) return cudaErrorInvalidValue;
     cudaError_t e;
@@ -1023,7 +1403,10 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     if ((e = c.slots.ensure((size_t)sh.total_px * 4)) != cudaSuccess) return e;
     if ((e = c.shadow.ensure((size_t)sh.total_px)) != cudaSuccess) return e;  // shadow states
     if ((e = c.hdr.ensure((size_t)sh.total_pyr * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = c.sched.ensure(((size_t)c.num_sms + 1) * 4)) != cudaSuccess) return e;
+    if ((e = c.sched.ensure(std::max<size_t>((size_t)c.num_sms + 1, 2 * FAN_COUNTERS + 1) * 4)) != cudaSuccess) return e;
+    bool shadows = false;  // some observer casts shadow rays
+    for (uint32_t i = 0; i < n; ++i)
+        shadows = shadows || (r.u[i].mode == 0u && r.u[i].shadow_mode != 0u && r.u[i].num_flashes == 0u);
     bool binned = false;
     if (!r.star_brute && sd.num_stars > 0)
         for (uint32_t i = 0; i < n; ++i) binned = binned || stars_binned_for(r.u[i], sd.num_stars);
@@ -1081,6 +1464,11 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     ws.root_max = make_float4(s.root_max[0], s.root_max[1], s.root_max[2], s.root_max[3]);
     ws.root_ref = s.root_ref;
     ws.empty = s.empty ? 1u : 0u;
+    ws.fan_box = s.fan_box.as<float4>();
+    ws.fan_ref = s.fan_ref.as<uint32_t>();
+    ws.fan_root = s.fan_root;
+    ws.leaf_bits = 0;
+    while (s.max_leaf >> ws.leaf_bits) ++ws.leaf_bits;
     unsigned long long* work = reinterpret_cast<unsigned long long*>(counters + 4);
     const uint32_t* tile_pre = c.lvl_pre.as<uint32_t>();
     const uint32_t* pix_pre = tile_pre + stride;
@@ -1107,8 +1495,8 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         ta.tile_pre = tile_pre;
         ta.n = n;
         ta.total_rays = sh.total_tiles * 32u;
-        ta.tile_w = t.tile_w;
-        ta.tile_h = t.tile_h;
+        ta.tile_w = tile_w;
+        ta.tile_h = tile_h;
         ta.hits = c.hits.as<float4>();
         ta.slots = c.slots.as<uint32_t>();
         ta.shadow = c.shadow.as<uint8_t>();
@@ -1124,6 +1512,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         ta.work = work;
         uint32_t blocks = (uint32_t)c.num_sms * t.blocks_per_sm;
         uint32_t need = (uint32_t)(((uint64_t)sh.total_tiles * 32 + t.block_threads - 1) / t.block_threads);
+        if (packet) need = blocks;  // a small frame's slow tiles are split among the warps that have none
         if (blocks > need) blocks = need;
         const size_t smem = t.leaf_coop ? (size_t)(t.block_threads / 32) * COOP_SMEM_PER_WARP : 0;
         const bool lean = !t.leaf_coop && t.leaf_batch == 1 && t.refill_lanes == 32 && t.chunk_tiles == 1;
@@ -1132,7 +1521,23 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
             const bool oct = s.copies == 16, top = oct && t.top_levels > 0;
             ta.top_n = top ? s.top_end[t.top_levels - 1] : 0u;
             const size_t ssm = lean_stack_bytes(t) + (size_t)ta.top_n * 72u;
-            launch_lean(t.stack_smem, r.count_work, oct, top, t.packet != 0, blocks, t.block_threads, ssm, st, ta);
+            if (packet) {
+                FanTasks ft;
+                ft.count = c.sched.as<uint32_t>();
+                ft.num_shadows = ft.count + 2 * FAN_COUNTERS;
+                ft.list = c.fan_list.as<uint32_t>();
+                ft.shadows = c.fan_shadows.as<uint32_t>();
+                ft.waste = sh.total_tiles < FAN_SMALL_TILES ? FAN_WASTE_SMALL : FAN_WASTE;
+                const uint32_t warps = t.block_threads / 32;
+                if (oct) k_fan_trace<true><<<blocks, t.block_threads, warps * sizeof(FanQueue), st>>>(ta, ft);
+                else k_fan_trace<false><<<blocks, t.block_threads, warps * sizeof(FanQueue), st>>>(ta, ft);
+                if (shadows) {
+                    ft.count += FAN_COUNTERS;
+                    k_fan_shadow<<<blocks, t.block_threads, warps * sizeof(FanShadows), st>>>(ta, ft);
+                }
+            } else {
+                launch_lean(t.stack_smem, r.count_work, oct, top, blocks, t.block_threads, ssm, st, ta);
+            }
         } else if (t.leaf_coop) {
             if (r.count_work) k_trace_batch<true, true><<<blocks, t.block_threads, smem, st>>>(ta);
             else k_trace_batch<false, true><<<blocks, t.block_threads, smem, st>>>(ta);
@@ -1255,7 +1660,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                        t.leaf_coop);
     key = mix(key, t.home_pct);
     key = mix(key, ((uint64_t)t.stack_smem << 32) | t.top_levels);
-    key = mix(key, t.packet);
+    key = mix(key, (packet ? 1u : 0u) | (shadows ? 2u : 0u));
     key = mix(key, binned ? 0x5354ull : 0ull);
     key = mix(key, simple ? 0x51ull : 0ull);
     for (auto& o : sh.obs) key = mix(key, ((uint64_t)o.width << 32) | o.height);

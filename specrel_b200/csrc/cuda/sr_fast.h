@@ -64,6 +64,9 @@ struct FastScene {
     DevMem boxes, refs, scratch;
     // Up links for the packet traversal's ordering of equal-lambda hits (WideScene::up / leafpar).
     DevMem up, leafpar;
+    // The packet walk's layout (sr_fan.cuh); fan_levels 0: none, the rays walk alone.
+    DevMem fan_box, fan_ref;
+    uint32_t fan_root = 0, fan_levels = 0, num_fans = 0;
     uint32_t num_wide = 0;
     uint32_t depth = 0;
     uint32_t root_ref = 0;
@@ -74,7 +77,7 @@ struct FastScene {
     uint32_t max_leaf = 0;  // most primitives in a leaf, as the last build saw
     uint32_t top_end[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // wide nodes in the top k + 1 levels (breadth-first prefix)
     float root_min[4] = {0, 0, 0, 0}, root_max[4] = {0, 0, 0, 0};
-    size_t bytes() const { return boxes.bytes + refs.bytes + up.bytes + leafpar.bytes; }
+    size_t bytes() const { return boxes.bytes + refs.bytes + up.bytes + leafpar.bytes + fan_box.bytes + fan_ref.bytes; }
 };
 
 // Per-observer description of a batch (device copy in BatchCtx::obs).
@@ -97,7 +100,8 @@ struct FastCtx {
     // Batch buffers, grown on demand.
     // shadow: one byte per pixel, the main light's shadow ray as traced (0 none, 1 clear, 2 occluded)
     // sched: the tile counters of the trace kernel, one per SM band then the shared pool's
-    DevMem U, cam64, cam, obs, lvl_pre, hits, slots, shadow, hdr, rgb, sched;
+    // fan_list, fan_shadows: the packet walk's queue, and its list of pixels that cast shadow rays
+    DevMem U, cam64, cam, obs, lvl_pre, hits, slots, shadow, hdr, rgb, sched, fan_list, fan_shadows;
     // Star binning: per (observer, star) cone events and tile rectangles; per 16x16 tile a count,
     // a list offset and a fill cursor; the lists; the prefix sum's scratch.
     DevMem star_cd, star_cu, star_rect, star_count, star_offset, star_fill, star_list, star_scan;

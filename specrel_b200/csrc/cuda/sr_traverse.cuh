@@ -63,6 +63,11 @@ struct WideScene {
     float4 root_min, root_max;
     uint32_t root_ref;    // packed reference of the root (a leaf, or wide node 0)
     uint32_t empty;       // no geometry at all
+    // The fan layout (sr_fan.cuh): per fan node 32 box minima, 32 maxima and 32 references.
+    const float4* fan_box;
+    const uint32_t* fan_ref;
+    uint32_t fan_root;
+    uint32_t leaf_bits;  // bits of the largest leaf's primitive count
 };
 
 // Traversal work of one thread (the SR_FLAG_COUNT_WORK variant only).
@@ -493,30 +498,6 @@ __device__ __forceinline__ bool any_lean(const WideScene& s, uint32_t cur, float
     }
 }
 
-// ---------------------------------------------------------------------------------------------
-// Packet traversal: the closest-hit queries of a warp's 32 lanes (the primary rays of one tile of
-// neighbouring pixels) walked as one. The warp steps through one node sequence. At an internal node
-// every lane that takes part tests both child boxes against its own ray, bounded by its own
-// closest hit so far; a child is entered when some lane enters it, and when lanes enter both, the
-// child that more of them enter first goes first (the left one on a tie), the other pushed with each
-// lane's entry parameter (+inf where the lane misses it) and taken again when some lane still
-// enters it before its closest hit. At a leaf every lane that takes part tests the records in
-// order. Rays of neighbouring pixels walk nearly the same nodes (on the 7.9M-tet workload the union
-// of a 4x8 tile's node visits is 6% above one ray's), so the warp runs one instruction stream with
-// warp-wide loads of one node or record, where the per-lane order runs the node and record code
-// side by side over lanes standing at different nodes.
-//
-// The result of each lane is closest_lean's. The closest hit so far is never nearer than the
-// reference's final one, so no box the reference enters on the way to its hit is culled, and that
-// hit is tested; no nearer hit exists among the records tested; of hits at equal lambda the lane
-// keeps the one the reference's near-first order meets first (packet_precedes). This holds as long
-// as every hit lies beyond the entry parameter of its leaf's box as computed. A hit's event passes
-// the barycentric test, so it lies inside the record's box, which the build pads by 1e-4: in ray
-// parameter a margin of 1e-4 / |d| on the entering axis, against a rounding of the computed entry
-// of order 1e-7 lambda; only hits far along a fast axis (lambda ~ 100 or more with |d| ~ 8) bring
-// the two within a factor of two.
-// ---------------------------------------------------------------------------------------------
-
 // Whether hot record a comes before hot record b in the reference's visiting order for this ray
 // (a != b): at their lowest common ancestor the near child (smaller entry parameter, the left one on
 // equal entries) is entered first; within one leaf, records in index order.
@@ -579,164 +560,6 @@ __device__ __noinline__ bool packet_precedes(const WideScene& s, uint32_t a, uin
     }
     const bool left_first = enl <= enr;
     return sa == 0 ? left_first : !left_first;
-}
-
-// The packet form of closest_lean for the whole warp (all 32 lanes call it together, converged).
-// `in`: this lane's ray enters the scene's box (the others take no part). Returns the slot or -1;
-// `t_max` ends as the closest hit's parameter.
-template <bool OCT, class Stack>
-__device__ __forceinline__ int closest_packet(const WideScene& s, bool in, float4 no, float4 d, float4 inv, float t_min,
-                                              float& t_max, GeomHit& best, const Stack& st, uint32_t* err) {
-    constexpr uint32_t FULL = 0xFFFFFFFFu;
-    const float none = __uint_as_float(0x7F800000u);  // +inf: the lane does not enter the pushed child
-    const float4* ob = OCT ? octant_boxes(s, inv) : s.boxes;
-    int slot = -1, sp = 0;
-    uint32_t visits = 0;
-    float t_below = __uint_as_float(__float_as_uint(t_max) - 1u);
-    uint32_t cur = s.root_ref;
-    for (;;) {
-        if (cur & REF_LEAF) {
-            const uint32_t k = cur & REF_FIRST_MASK;
-            if (in) {
-                GeomHit gh;
-                // Hits up to and including t_max, so that a hit at the closest hit's lambda is seen.
-                if (intersect_lean(s.geoms + 5u * k, no, d, t_min, __uint_as_float(__float_as_uint(t_max) + 1u), &gh)) {
-                    if (gh.lambda < t_max) {
-                        t_max = gh.lambda;
-                        t_below = __uint_as_float(__float_as_uint(t_max) - 1u);
-                        best = gh;
-                        slot = (int)k;
-                    } else if (slot >= 0 && packet_precedes<OCT>(s, k, (uint32_t)slot, no, inv, t_min, err)) {
-                        best = gh;
-                        slot = (int)k;
-                    }
-                }
-            }
-            cur += REF_NEXT_PRIM;
-            if (cur & REF_COUNT_MASK) continue;
-        } else {
-            if (++visits > MAX_VISITS_FAST) {
-                atomicOr(err, ERR_TRAVERSAL_LIMIT);
-                break;
-            }
-            const uint2 r = __ldg(s.refs + cur);
-            // Every lane computes (the warp runs the code once either way); lanes that take no part
-            // are masked out, so the step has no divergent branch.
-            const float4* b = ob + 4ull * cur;
-            const float4 lnear = __ldg(b), lfar = __ldg(b + 1), rnear = __ldg(b + 2), rfar = __ldg(b + 3);
-            float enl, exl, enr, exr;
-            if (OCT) {
-                slab_octant(lnear, lfar, no, inv, t_min, t_below, &enl, &exl);
-                slab_octant(rnear, rfar, no, inv, t_min, t_below, &enr, &exr);
-            } else {
-                slab_interval(lnear, lfar, no, inv, t_min, t_below, &enl, &exl);
-                slab_interval(rnear, rfar, no, inv, t_min, t_below, &enr, &exr);
-            }
-            const bool hl = in && exl >= enl;  // and enl < t_max
-            const bool hr = in && exr >= enr;
-            const uint32_t ml = __ballot_sync(FULL, hl), mr = __ballot_sync(FULL, hr);
-            if (ml && mr) {
-                const uint32_t nl = __popc(__ballot_sync(FULL, hl && (!hr || enl <= enr)));
-                const bool left_first = 2u * nl >= (uint32_t)__popc(ml | mr);
-                if (sp < FAST_STACK)
-                    st.put(sp++, left_first ? make_uint2(r.y, __float_as_uint(hr ? enr : none))
-                                            : make_uint2(r.x, __float_as_uint(hl ? enl : none)));
-                else atomicOr(err, ERR_BAD_INDEX);
-                cur = left_first ? r.x : r.y;
-                in = left_first ? hl : hr;
-                continue;
-            }
-            if (ml | mr) {
-                cur = ml ? r.x : r.y;
-                in = ml ? hl : hr;
-                continue;
-            }
-        }
-        bool found = false;
-        while (sp > 0) {
-            const uint2 e = st.get(--sp);
-            const bool take = __uint_as_float(e.y) < t_max;
-            if (__any_sync(FULL, take)) {
-                cur = e.x;
-                in = take;
-                found = true;
-                break;
-            }
-        }
-        if (!found) break;
-    }
-    return slot;
-}
-
-// The packet form of any_lean for the whole warp (all 32 lanes call it together, converged): the
-// lanes' any-hit queries walked as one node sequence, left child first. A lane takes part in a
-// node or leaf its own ray enters, and stops once it has a hit; the walk ends when no lane still
-// searching takes part in anything left. Every lane tests records of leaves its ray enters until
-// one hits, so its answer is any_lean's (an any-hit answer does not depend on the order).
-// `in`: this lane has a query whose ray enters the scene's box.
-template <bool OCT, class Stack>
-__device__ __forceinline__ bool any_packet(const WideScene& s, bool in, float4 no, float4 d, float4 inv, float t_min,
-                                           float t_max, const Stack& st, uint32_t* err) {
-    constexpr uint32_t FULL = 0xFFFFFFFFu;
-    const float4* ob = OCT ? octant_boxes(s, inv) : s.boxes;
-    bool hit = false, part = in;
-    int sp = 0;
-    uint32_t visits = 0;
-    uint32_t cur = s.root_ref;
-    for (;;) {
-        if (cur & REF_LEAF) {
-            if (part && !hit) {
-                GeomHit gh;
-                hit = intersect_lean(s.geoms + 5u * (cur & REF_FIRST_MASK), no, d, t_min, t_max, &gh);
-            }
-            cur += REF_NEXT_PRIM;
-            if ((cur & REF_COUNT_MASK) && __any_sync(FULL, part && !hit)) continue;
-        } else {
-            if (++visits > MAX_VISITS_FAST) {
-                atomicOr(err, ERR_TRAVERSAL_LIMIT);
-                break;
-            }
-            const uint2 r = __ldg(s.refs + cur);
-            const float4* b = ob + 4ull * cur;
-            const float4 lnear = __ldg(b), lfar = __ldg(b + 1), rnear = __ldg(b + 2), rfar = __ldg(b + 3);
-            float enl, exl, enr, exr;
-            if (OCT) {
-                slab_octant(lnear, lfar, no, inv, t_min, t_max, &enl, &exl);
-                slab_octant(rnear, rfar, no, inv, t_min, t_max, &enr, &exr);
-            } else {
-                slab_interval(lnear, lfar, no, inv, t_min, t_max, &enl, &exl);
-                slab_interval(rnear, rfar, no, inv, t_min, t_max, &enr, &exr);
-            }
-            const bool live = part && !hit;
-            const bool hl = live && exl >= enl, hr = live && exr >= enr;
-            const uint32_t ml = __ballot_sync(FULL, hl), mr = __ballot_sync(FULL, hr);
-            if (ml && mr) {
-                if (sp < FAST_STACK) st.put(sp++, make_uint2(r.y, hr ? 1u : 0u));
-                else atomicOr(err, ERR_BAD_INDEX);
-                cur = r.x;
-                part = hl;
-                continue;
-            }
-            if (ml | mr) {
-                cur = ml ? r.x : r.y;
-                part = ml ? hl : hr;
-                continue;
-            }
-        }
-        bool found = false;
-        while (sp > 0) {
-            const uint2 e = st.get(--sp);
-            const bool take = e.y != 0u && !hit;
-            if (__any_sync(FULL, take)) {
-                cur = e.x;
-                part = take;
-                found = true;
-                break;
-            }
-        }
-        if (!found) break;
-    }
-    return hit;
 }
 
 }  // namespace srk
