@@ -3,6 +3,8 @@
 // exactly the operations, in exactly the order, of the forward shading code they mirror, so they
 // reproduce the forward frame's values bit for bit; the derivative parts follow the chain rule.
 // Min/max/clamp select by value and carry the selected operand's derivatives (zero for a constant).
+// Templated on the number of tangents: all seven in one thread, or one per thread (a group of threads then holds
+// a number's tangents, each computing the value too), with the same operations per tangent either way.
 // The types live in their own namespace so that their overloads never hide the float ones.
 #pragma once
 #include "sr_device.cuh"
@@ -13,164 +15,210 @@ using srd::F3;
 
 constexpr int NT = 7;  // tangents
 
-struct DF {
+template <int N>
+struct DFT {
     float v;
-    float d[NT];
+    float d[N];
 };
+using DF = DFT<NT>;
 
-__device__ __forceinline__ DF dconst(float v) {
-    DF r;
+template <int N = NT>
+__device__ __forceinline__ DFT<N> dconst(float v) {
+    DFT<N> r;
     r.v = v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = 0.0f;
+    for (int i = 0; i < N; ++i) r.d[i] = 0.0f;
     return r;
 }
-__device__ __forceinline__ DF operator+(const DF& a, const DF& b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator+(const DFT<N>& a, const DFT<N>& b) {
+    DFT<N> r;
     r.v = a.v + b.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] + b.d[i];
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] + b.d[i];
     return r;
 }
-__device__ __forceinline__ DF operator-(const DF& a, const DF& b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator-(const DFT<N>& a, const DFT<N>& b) {
+    DFT<N> r;
     r.v = a.v - b.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] - b.d[i];
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] - b.d[i];
     return r;
 }
-__device__ __forceinline__ DF operator-(const DF& a) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator-(const DFT<N>& a) {
+    DFT<N> r;
     r.v = -a.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = -a.d[i];
+    for (int i = 0; i < N; ++i) r.d[i] = -a.d[i];
     return r;
 }
-__device__ __forceinline__ DF operator*(const DF& a, const DF& b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator*(const DFT<N>& a, const DFT<N>& b) {
+    DFT<N> r;
     r.v = a.v * b.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] * b.v + a.v * b.d[i];
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * b.v + a.v * b.d[i];
     return r;
 }
-__device__ __forceinline__ DF operator/(const DF& a, const DF& b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator/(const DFT<N>& a, const DFT<N>& b) {
+    DFT<N> r;
     r.v = a.v / b.v;
     const float ib = 1.0f / b.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) * ib;
+    for (int i = 0; i < N; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) * ib;
     return r;
 }
-__device__ __forceinline__ DF operator+(const DF& a, float b) {
-    DF r = a;
+template <int N>
+__device__ __forceinline__ DFT<N> operator+(const DFT<N>& a, float b) {
+    DFT<N> r = a;
     r.v = a.v + b;
     return r;
 }
-__device__ __forceinline__ DF operator+(float a, const DF& b) {
-    DF r = b;
+template <int N>
+__device__ __forceinline__ DFT<N> operator+(float a, const DFT<N>& b) {
+    DFT<N> r = b;
     r.v = a + b.v;
     return r;
 }
-__device__ __forceinline__ DF operator-(const DF& a, float b) {
-    DF r = a;
+template <int N>
+__device__ __forceinline__ DFT<N> operator-(const DFT<N>& a, float b) {
+    DFT<N> r = a;
     r.v = a.v - b;
     return r;
 }
-__device__ __forceinline__ DF operator-(float a, const DF& b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator-(float a, const DFT<N>& b) {
+    DFT<N> r;
     r.v = a - b.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = -b.d[i];
+    for (int i = 0; i < N; ++i) r.d[i] = -b.d[i];
     return r;
 }
-__device__ __forceinline__ DF operator*(const DF& a, float s) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator*(const DFT<N>& a, float s) {
+    DFT<N> r;
     r.v = a.v * s;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] * s;
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * s;
     return r;
 }
-__device__ __forceinline__ DF operator*(float s, const DF& a) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator*(float s, const DFT<N>& a) {
+    DFT<N> r;
     r.v = s * a.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = s * a.d[i];
+    for (int i = 0; i < N; ++i) r.d[i] = s * a.d[i];
     return r;
 }
-__device__ __forceinline__ DF operator/(const DF& a, float b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator/(const DFT<N>& a, float b) {
+    DFT<N> r;
     r.v = a.v / b;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] / b;
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] / b;
     return r;
 }
-__device__ __forceinline__ DF operator/(float a, const DF& b) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> operator/(float a, const DFT<N>& b) {
+    DFT<N> r;
     r.v = a / b.v;
     const float ib = 1.0f / b.v;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = -r.v * b.d[i] * ib;
+    for (int i = 0; i < N; ++i) r.d[i] = -r.v * b.d[i] * ib;
     return r;
 }
-__device__ __forceinline__ DF dsqrt(const DF& a) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> dsqrt(const DFT<N>& a) {
+    DFT<N> r;
     r.v = sqrtf(a.v);
     const float k = r.v > 0.0f ? 0.5f / r.v : 0.0f;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] * k;
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * k;
     return r;
 }
-__device__ __forceinline__ DF dexp(const DF& a) {
-    DF r;
+template <int N>
+__device__ __forceinline__ DFT<N> dexp(const DFT<N>& a) {
+    DFT<N> r;
     r.v = expf(a.v);
 #pragma unroll
-    for (int i = 0; i < NT; ++i) r.d[i] = a.d[i] * r.v;
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * r.v;
     return r;
 }
 // fmaxf(a, b) / fminf(a, b) with a constant b.
-__device__ __forceinline__ DF dmaxc(const DF& a, float b) { return fmaxf(a.v, b) == a.v && a.v >= b ? a : dconst(fmaxf(a.v, b)); }
-__device__ __forceinline__ DF dminc(const DF& a, float b) { return fminf(a.v, b) == a.v && a.v <= b ? a : dconst(fminf(a.v, b)); }
-__device__ __forceinline__ DF dclamp(const DF& x, float lo, float hi) {  // clampf_
-    if (x.v < lo) return dconst(lo);
-    if (x.v > hi) return dconst(hi);
+template <int N>
+__device__ __forceinline__ DFT<N> dmaxc(const DFT<N>& a, float b) { return fmaxf(a.v, b) == a.v && a.v >= b ? a : dconst<N>(fmaxf(a.v, b)); }
+template <int N>
+__device__ __forceinline__ DFT<N> dminc(const DFT<N>& a, float b) { return fminf(a.v, b) == a.v && a.v <= b ? a : dconst<N>(fminf(a.v, b)); }
+template <int N>
+__device__ __forceinline__ DFT<N> dclamp(const DFT<N>& x, float lo, float hi) {  // clampf_
+    if (x.v < lo) return dconst<N>(lo);
+    if (x.v > hi) return dconst<N>(hi);
     return x;
 }
 
-struct DF3 {
-    DF x, y, z;
+template <int N>
+struct DF3T {
+    DFT<N> x, y, z;
 };
-struct DF4 {
-    DF x, y, z, w;  // (t, x, y, z)
+template <int N>
+struct DF4T {
+    DFT<N> x, y, z, w;  // (t, x, y, z)
 };
+using DF3 = DF3T<NT>;
+using DF4 = DF4T<NT>;
 
-__device__ __forceinline__ DF4 dconst4(float4 a) { return DF4{dconst(a.x), dconst(a.y), dconst(a.z), dconst(a.w)}; }
-__device__ __forceinline__ float4 val4(const DF4& a) { return make_float4(a.x.v, a.y.v, a.z.v, a.w.v); }
-__device__ __forceinline__ DF4 add4(const DF4& a, const DF4& b) { return DF4{a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w}; }
-__device__ __forceinline__ DF4 sub4(const DF4& a, const DF4& b) { return DF4{a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w}; }
-__device__ __forceinline__ DF4 sub4(float4 a, const DF4& b) { return DF4{a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w}; }
-__device__ __forceinline__ DF4 mul4(const DF4& a, const DF& s) { return DF4{a.x * s, a.y * s, a.z * s, a.w * s}; }
-__device__ __forceinline__ DF4 mul4(const DF4& a, float s) { return DF4{a.x * s, a.y * s, a.z * s, a.w * s}; }
-__device__ __forceinline__ DF4 mul4(float4 a, const DF& s) { return DF4{a.x * s, a.y * s, a.z * s, a.w * s}; }
-__device__ __forceinline__ DF4 neg4(const DF4& a) { return DF4{-a.x, -a.y, -a.z, -a.w}; }
+template <int N = NT>
+__device__ __forceinline__ DF4T<N> dconst4(float4 a) { return DF4T<N>{dconst<N>(a.x), dconst<N>(a.y), dconst<N>(a.z), dconst<N>(a.w)}; }
+template <int N>
+__device__ __forceinline__ float4 val4(const DF4T<N>& a) { return make_float4(a.x.v, a.y.v, a.z.v, a.w.v); }
+template <int N>
+__device__ __forceinline__ DF4T<N> add4(const DF4T<N>& a, const DF4T<N>& b) { return DF4T<N>{a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w}; }
+template <int N>
+__device__ __forceinline__ DF4T<N> sub4(const DF4T<N>& a, const DF4T<N>& b) { return DF4T<N>{a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w}; }
+template <int N>
+__device__ __forceinline__ DF4T<N> sub4(float4 a, const DF4T<N>& b) { return DF4T<N>{a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w}; }
+template <int N>
+__device__ __forceinline__ DF4T<N> mul4(const DF4T<N>& a, const DFT<N>& s) { return DF4T<N>{a.x * s, a.y * s, a.z * s, a.w * s}; }
+template <int N>
+__device__ __forceinline__ DF4T<N> mul4(const DF4T<N>& a, float s) { return DF4T<N>{a.x * s, a.y * s, a.z * s, a.w * s}; }
+template <int N>
+__device__ __forceinline__ DF4T<N> mul4(float4 a, const DFT<N>& s) { return DF4T<N>{a.x * s, a.y * s, a.z * s, a.w * s}; }
+template <int N>
+__device__ __forceinline__ DF4T<N> neg4(const DF4T<N>& a) { return DF4T<N>{-a.x, -a.y, -a.z, -a.w}; }
 // mdot / edot in the forward code's order.
-__device__ __forceinline__ DF mdot(const DF4& a, const DF4& b) { return -a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
-__device__ __forceinline__ DF mdot(const DF4& a, float4 b) { return -a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
-__device__ __forceinline__ DF edot(float4 a, const DF4& b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
-__device__ __forceinline__ DF3 spatial(const DF4& a) { return DF3{a.y, a.z, a.w}; }
-__device__ __forceinline__ DF dot3(const DF3& a, const DF3& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ DF3 add(const DF3& a, const DF3& b) { return DF3{a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ DF3 mul(const DF3& a, const DF& s) { return DF3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ DF3 mul(F3 a, const DF& s) { return DF3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ DF3 mulv(const DF3& a, F3 b) { return DF3{a.x * b.x, a.y * b.y, a.z * b.z}; }
-__device__ __forceinline__ DF3 dconst3(F3 a) { return DF3{dconst(a.x), dconst(a.y), dconst(a.z)}; }
-__device__ __forceinline__ DF len3(const DF3& a) { return dsqrt(dot3(a, a)); }
-__device__ __forceinline__ DF3 normalized3(const DF3& a) {
-    DF l = len3(a);
+template <int N>
+__device__ __forceinline__ DFT<N> mdot(const DF4T<N>& a, const DF4T<N>& b) { return -a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+template <int N>
+__device__ __forceinline__ DFT<N> mdot(const DF4T<N>& a, float4 b) { return -a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+template <int N>
+__device__ __forceinline__ DFT<N> edot(float4 a, const DF4T<N>& b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+template <int N>
+__device__ __forceinline__ DF3T<N> spatial(const DF4T<N>& a) { return DF3T<N>{a.y, a.z, a.w}; }
+template <int N>
+__device__ __forceinline__ DFT<N> dot3(const DF3T<N>& a, const DF3T<N>& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+template <int N>
+__device__ __forceinline__ DF3T<N> add(const DF3T<N>& a, const DF3T<N>& b) { return DF3T<N>{a.x + b.x, a.y + b.y, a.z + b.z}; }
+template <int N>
+__device__ __forceinline__ DF3T<N> mul(const DF3T<N>& a, const DFT<N>& s) { return DF3T<N>{a.x * s, a.y * s, a.z * s}; }
+template <int N>
+__device__ __forceinline__ DF3T<N> mul(F3 a, const DFT<N>& s) { return DF3T<N>{a.x * s, a.y * s, a.z * s}; }
+template <int N>
+__device__ __forceinline__ DF3T<N> mulv(const DF3T<N>& a, F3 b) { return DF3T<N>{a.x * b.x, a.y * b.y, a.z * b.z}; }
+template <int N = NT>
+__device__ __forceinline__ DF3T<N> dconst3(F3 a) { return DF3T<N>{dconst<N>(a.x), dconst<N>(a.y), dconst<N>(a.z)}; }
+template <int N>
+__device__ __forceinline__ DFT<N> len3(const DF3T<N>& a) { return dsqrt(dot3(a, a)); }
+template <int N>
+__device__ __forceinline__ DF3T<N> normalized3(const DF3T<N>& a) {
+    DFT<N> l = len3(a);
     if (l.v > 1e-12f) {
-        DF il = 1.0f / l;
-        return DF3{a.x * il, a.y * il, a.z * il};
+        DFT<N> il = 1.0f / l;
+        return DF3T<N>{a.x * il, a.y * il, a.z * il};
     }
-    return DF3{dconst(0.0f), dconst(0.0f), dconst(0.0f)};
+    return DF3T<N>{dconst<N>(0.0f), dconst<N>(0.0f), dconst<N>(0.0f)};
 }
 
 // A double with its derivatives with respect to the three rapidity components, for the FP64

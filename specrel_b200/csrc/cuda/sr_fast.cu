@@ -1418,7 +1418,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
             (ui.mode == 0u && sd.num_stars > 0u && !(binned && stars_binned_for(ui, sd.num_stars))))
             simple = false;
     }
-    const size_t old_star = c.star_cd.bytes + c.star_rect.bytes + c.star_count.bytes + c.star_list.bytes + c.star_scan.bytes;
+    const size_t old_star = c.star_r.bytes + c.star_box.bytes + c.star_count.bytes + c.star_list.bytes + c.star_scan.bytes;
     // Star lists: room for every (observer, star) in 8 tiles; tiles past the room sum every star.
     const uint32_t list_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(8ull * n * sd.num_stars, 1u << 20), 1u << 30);
     size_t scan_bytes = 0;
@@ -1426,16 +1426,16 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         const size_t pairs = (size_t)n * sd.num_stars;
         const size_t tiles = sh.total_star_tiles;
         cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)tiles, st);
-        if ((e = c.star_cd.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
-        if ((e = c.star_cu.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
-        if ((e = c.star_rect.ensure(pairs * sizeof(uint4))) != cudaSuccess) return e;
+        if ((e = c.star_r.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
+        if ((e = c.star_color.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
+        if ((e = c.star_box.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
         if ((e = c.star_count.ensure(tiles * 4)) != cudaSuccess) return e;
         if ((e = c.star_offset.ensure(tiles * 4)) != cudaSuccess) return e;
         if ((e = c.star_fill.ensure(tiles * 4)) != cudaSuccess) return e;
         if ((e = c.star_list.ensure((size_t)list_cap * 4)) != cudaSuccess) return e;
         if ((e = c.star_scan.ensure(scan_bytes)) != cudaSuccess) return e;
     }
-    if (c.star_cd.bytes + c.star_rect.bytes + c.star_count.bytes + c.star_list.bytes + c.star_scan.bytes != old_star)
+    if (c.star_r.bytes + c.star_box.bytes + c.star_count.bytes + c.star_list.bytes + c.star_scan.bytes != old_star)
         fast_release(c);
     if (!r.rgb && (e = c.rgb.ensure((size_t)sh.total_px * 4)) != cudaSuccess) return e;
     if ((e = c.hU.ensure(n * sizeof(SrGpuUniforms))) != cudaSuccess) return e;
@@ -1588,9 +1588,10 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
             ba.stars = sd.stars;
             ba.n = n;
             ba.num_stars = sd.num_stars;
-            ba.cd = c.star_cd.as<float4>();
-            ba.cu = c.star_cu.as<float4>();
-            ba.rect = c.star_rect.as<uint4>();
+            ba.r = c.star_r.as<float4>();
+            ba.color = c.star_color.as<float4>();
+            ba.box = c.star_box.as<float4>();
+            ba.bb = bb;
             ba.count = c.star_count.as<uint32_t>();
             ba.offset = c.star_offset.as<uint32_t>();
             ba.fill = c.star_fill.as<uint32_t>();
@@ -1604,6 +1605,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                 cudaSuccess)
                 return x;
             k_star_fill<<<gb, 256, 0, st>>>(ba);
+            k_star_sort<<<(uint32_t)tiles, 256, STAR_SORT_CAP * 4, st>>>(ba.count, ba.offset, ba.list, list_cap, sd.num_stars);
             StarTileArgs ta2;
             ta2.s = sd;
             ta2.U = sa.U;
@@ -1613,18 +1615,20 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
             ta2.n = n;
             ta2.hits = sa.hits;
             ta2.slots = sa.slots;
-            ta2.cd = ba.cd;
-            ta2.cu = ba.cu;
+            ta2.r = ba.r;
+            ta2.color = ba.color;
+            ta2.box = ba.box;
             ta2.count = ba.count;
             ta2.offset = ba.offset;
             ta2.list = ba.list;
             ta2.list_cap = list_cap;
             ta2.hdr = sa.hdr;
             ta2.bb = bb;
-            k_star_tiles<<<(uint32_t)tiles, 256, STAR_SORT_CAP * 4, st>>>(ta2);
+            k_star_tiles<<<(uint32_t)tiles * STAR_BLOCKS, 64, 0, st>>>(ta2);
             if ((x = cudaGetLastError()) != cudaSuccess) return x;
         }
         if (timed) cudaEventRecord(r.ev[3], st);
+        if (r.no_image) return cudaSuccess;
         for (int k = 1; k <= SR_BLOOM_LEVELS; ++k) {
             const uint32_t* pre = tile_pre + (size_t)(1 + k) * stride;
             uint32_t tot = sh.pre[(size_t)(1 + k) * stride + n];
@@ -1662,7 +1666,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     key = mix(key, ((uint64_t)t.stack_smem << 32) | t.top_levels);
     key = mix(key, (packet ? 1u : 0u) | (shadows ? 2u : 0u));
     key = mix(key, binned ? 0x5354ull : 0ull);
-    key = mix(key, simple ? 0x51ull : 0ull);
+    key = mix(key, (simple ? 0x51ull : 0ull) | (r.no_image ? 0x100ull : 0ull));
     for (auto& o : sh.obs) key = mix(key, ((uint64_t)o.width << 32) | o.height);
     auto it = c.graphs.find(key);
     if (it == c.graphs.end()) {
@@ -1705,7 +1709,8 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
         br.n = 1;
         br.u = &u;
         br.cam64 = &cam;
-        br.use_graph = false;
+        br.use_graph = true;
+        br.no_image = true;
         c.adj_valid = false;
         if ((e = fast_render_batch(c, s, t, sd, anchor, bb, counters, br, st)) != cudaSuccess) return e;
     }
@@ -1733,7 +1738,9 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     if ((e = c.adj_weight.ensure(2 * npx * 3 * sizeof(double))) != cudaSuccess) return e;
     if ((e = c.adj_grid.ensure(npx)) != cudaSuccess) return e;
     if ((e = c.adj_hdr.ensure(npx * sizeof(float4))) != cudaSuccess) return e;
-    if (stars_on && (e = c.adj_stars.ensure((size_t)sd.num_stars * sizeof(DF4))) != cudaSuccess) return e;
+    if (stars_on && (e = c.adj_stars.ensure((size_t)sd.num_stars * ADJ_STAR * sizeof(float))) != cudaSuccess) return e;
+    if (stars_on && (e = c.adj_star_sum.ensure(npx * ADJ_SUM * sizeof(float))) != cudaSuccess) return e;
+    if (stars_on && (e = c.adj_star_n.ensure(npx * 4)) != cudaSuccess) return e;
     if (stars_on && (e = c.adj_pass.ensure(list_cap * 32)) != cudaSuccess) return e;
     float4* pyr = c.adj_pyr.as<float4>();  // image levels 0..level
     float4* tpyr = pyr + loff[level + 1];  // target levels 0..level
@@ -1743,20 +1750,21 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     // The loss at the chosen level of `image` against the target, and (gradient mode) its weights
     // on the full image.
     auto loss_pass = [&](const void* image) -> cudaError_t {
-        cudaError_t x;
-        if ((x = cudaMemcpyAsync(pyr, image, npx * sizeof(float4), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return x;
-        if ((x = cudaMemcpyAsync(tpyr, target, npx * sizeof(float4), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return x;
+        // Level 0 is the image and the target themselves.
+        auto at = [&](const float4* level0, float4* levels, uint32_t k) { return k ? (const float4*)(levels + loff[k]) : level0; };
+        const float4* img0 = reinterpret_cast<const float4*>(image);
+        const float4* tgt0 = reinterpret_cast<const float4*>(target);
         for (uint32_t k = 1; k <= level; ++k) {
-            const dim3 g2((lw[k] + 15) / 16, (lh[k] + 15) / 16);
-            k_adj_down<<<g2, b2, 0, st>>>(pyr + loff[k - 1], lw[k - 1], lh[k - 1], pyr + loff[k], lw[k], lh[k]);
-            k_adj_down<<<g2, b2, 0, st>>>(tpyr + loff[k - 1], lw[k - 1], lh[k - 1], tpyr + loff[k], lw[k], lh[k]);
+            const dim3 g2((lw[k] + 15) / 16, (lh[k] + 15) / 16, 2);
+            k_adj_down<<<g2, b2, 0, st>>>(at(img0, pyr, k - 1), at(tgt0, tpyr, k - 1), lw[k - 1], lh[k - 1], pyr + loff[k],
+                                         tpyr + loff[k], lw[k], lh[k]);
         }
         const size_t nl = (size_t)lw[level] * lh[level];
         double* gl = (level % 2 == 0) ? g0 : g1;  // ends in g0 after `level` transposes
         const uint32_t lblocks = (uint32_t)((nl + 255) / 256);
-        k_adj_residual<<<lblocks, 256, 0, st>>>(pyr + loff[level], tpyr + loff[level], (uint32_t)nl, lw[level], row0,
+        k_adj_residual<<<lblocks, 256, 0, st>>>(at(img0, pyr, level), at(tgt0, tpyr, level), (uint32_t)nl, lw[level], row0,
                                                  row1, gl, c.adj_partials.as<double>());
-        k_adjoint_reduce<<<1, 256, 0, st>>>(c.adj_partials.as<double>(), lblocks, c.adj_out.as<double>() + ADJ_SLOTS);
+        k_adjoint_reduce<<<ADJ_SLOTS, 256, 0, st>>>(c.adj_partials.as<double>(), lblocks, c.adj_out.as<double>() + ADJ_SLOTS);
         for (uint32_t k = level; k >= 1; --k) {
             double* src = (k % 2 == 0) ? g0 : g1;
             double* dst = (k % 2 == 0) ? g1 : g0;
@@ -1772,8 +1780,8 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     // The duals of the camera and of the stars' cone events, then the pixels.
     k_adjoint_camera<<<1, 1, 0, st>>>(cam, anchor[0], anchor[1], anchor[2], anchor[3], c.adj_cam.as<DCam>());
     if (stars_on)
-        k_adjoint_stars<<<(sd.num_stars + 127) / 128, 128, 0, st>>>(sd.stars, sd.num_stars, c.adj_cam.as<DCam>(),
-                                                                  c.adj_stars.as<DF4>());
+        k_adjoint_stars<<<(sd.num_stars + 127) / 128, 128, 0, st>>>(sd.stars, sd.num_stars, c.star_box.as<float4>(),
+                                                                  c.adj_cam.as<DCam>(), bb, c.adj_stars.as<float>());
     AdjointArgs a;
     a.s = sd;
     a.U = c.U.as<SrGpuUniforms>();
@@ -1783,8 +1791,10 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     a.hits = c.hits.as<float4>();
     a.slots = c.slots.as<uint32_t>();
     a.shadow = c.shadow.as<uint8_t>();
-    a.star_dcd = stars_on ? c.adj_stars.as<DF4>() : nullptr;
-    a.star_cu = stars_on ? c.star_cu.as<float4>() : nullptr;
+    a.star = stars_on ? c.adj_stars.as<float>() : nullptr;
+    a.star_box = stars_on ? c.star_box.as<float4>() : nullptr;
+    a.star_sum = stars_on ? c.adj_star_sum.as<float>() : nullptr;
+    a.star_n = stars_on ? c.adj_star_n.as<uint32_t>() : nullptr;
     a.count = stars_on ? c.star_count.as<uint32_t>() : nullptr;
     a.offset = stars_on ? c.star_offset.as<uint32_t>() : nullptr;
     a.list = stars_on ? c.star_list.as<uint32_t>() : nullptr;
@@ -1805,8 +1815,9 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     const uint32_t ty0 = a.y0 / STAR_TILE, ty1 = (a.y1 + STAR_TILE - 1) / STAR_TILE;
     a.tile0 = ty0 * tx16;
     const uint32_t band_tiles = (ty1 - ty0) * tx16;
-    if (band_tiles) k_adjoint_pixels<<<band_tiles, 256, STAR_SORT_CAP * 4, st>>>(a);
-    k_adjoint_reduce<<<1, 256, 0, st>>>(a.partials, band_tiles, c.adj_out.as<double>());
+    if (band_tiles && stars_on) k_adjoint_star_sums<<<band_tiles * ADJ_STAR_BLOCKS, 256, 0, st>>>(a);
+    if (band_tiles) k_adjoint_pixels<<<band_tiles, 256, 0, st>>>(a);
+    k_adjoint_reduce<<<ADJ_SLOTS, 256, 0, st>>>(a.partials, band_tiles, c.adj_out.as<double>());
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (frozen && (e = loss_pass(c.adj_hdr.p)) != cudaSuccess) return e;
     double both[2 * ADJ_SLOTS];

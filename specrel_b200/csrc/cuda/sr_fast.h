@@ -102,11 +102,12 @@ struct FastCtx {
     // sched: the tile counters of the trace kernel, one per SM band then the shared pool's
     // fan_list, fan_shadows: the packet walk's queue, and its list of pixels that cast shadow rays
     DevMem U, cam64, cam, obs, lvl_pre, hits, slots, shadow, hdr, rgb, sched, fan_list, fan_shadows;
-    // Star binning: per (observer, star) cone events and tile rectangles; per 16x16 tile a count,
-    // a list offset and a fill cursor; the lists; the prefix sum's scratch.
-    DevMem star_cd, star_cu, star_rect, star_count, star_offset, star_fill, star_list, star_scan;
+    // Star binning: per (observer, star) the event in the observer's space, the colour and the footprint's box;
+    // per 16x16 tile a count, a list offset and a fill cursor; the lists; the prefix sum's scratch.
+    DevMem star_r, star_color, star_box, star_count, star_offset, star_fill, star_list, star_scan;
     // Gradient: the camera and the stars' cone events as duals, per-block partial sums, the result.
-    DevMem adj_cam, adj_stars, adj_partials, adj_out, adj_pyr, adj_weight, adj_grid, adj_pass, adj_hdr;
+    // adj_star_sum, adj_star_n: per pixel the star sum's duals and how many terms it has.
+    DevMem adj_cam, adj_stars, adj_partials, adj_out, adj_pyr, adj_weight, adj_grid, adj_pass, adj_hdr, adj_star_sum, adj_star_n;
     // The outcomes of the last gradient call (hits, shadows, star lists, grid lines, cut passes)
     // stay valid for frozen evaluations while no other frame is rendered.
     bool adj_valid = false;
@@ -139,6 +140,7 @@ struct BatchRequest {
     bool count_work;
     bool use_graph;
     bool star_brute;              // sum every star per pixel (no binning), as the reference
+    bool no_image;                // only the HDR image is wanted: no bloom, no packed pixels
     cudaEvent_t* ev;              // optional: 5 events, after camera, trace, shading, stars, bloom
 };
 cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd,
