@@ -560,14 +560,15 @@ class Engine:
         doubles, direction, t_min, t_max) on the device. Returns a structured array of SrRayHit."""
         r = np.atleast_2d(np.asarray(rays, np.float64))
         n = len(r)
-        arr = (_lib.Ray * max(n, 1))()
-        for i in range(n):
-            arr[i].origin[:] = list(r[i, 0:4])
-            arr[i].dir[:] = list(np.float32(r[i, 4:8]))
-            arr[i].t_min, arr[i].t_max = float(np.float32(r[i, 8])), float(np.float32(r[i, 9]))
-        out = (_lib.RayHit * max(n, 1))()
-        _check(self.L.sr_trace_rays(self.h, idx, arr, n, out), self.h, "trace_rays")
-        return np.ctypeslib.as_array(out)[:n].copy()
+        if n and (r.ndim != 2 or r.shape[1] < 8):
+            raise ValueError("rays: n x 10 values")
+        arr = np.zeros(max(n, 1), np.dtype(_lib.Ray))
+        if n:
+            arr["origin"][:n], arr["dir"][:n] = r[:, 0:4], r[:, 4:8]
+            arr["t_min"][:n], arr["t_max"][:n] = r[:, 8], r[:, 9]
+        out = np.zeros(max(n, 1), np.dtype(_lib.RayHit))
+        _check(self.L.sr_trace_rays(self.h, idx, arr.ctypes.data, n, out.ctypes.data), self.h, "trace_rays")
+        return out[:n]
 
     def tuning(self, idx: int) -> _lib.Tuning:
         t = _lib.Tuning()

@@ -73,6 +73,7 @@ struct sr_ctx {
     std::string last_error;
     std::string name;
     sre::DevBuf tables, counters, cam;
+    sre::DevBuf rays_in, rays_out;  // sr_trace_rays' buffers, kept up to RAY_BUFFER_KEEP rays
     srk::BBConst bb{};
     std::vector<std::unique_ptr<sre::SceneSlot>> scenes;
     sre::Frame frame;

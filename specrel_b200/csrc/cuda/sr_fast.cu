@@ -22,6 +22,7 @@
 
 #include "sr_camera.cuh"
 #include "sr_fast.h"
+#include "sr_ref.cuh"
 #include "sr_shade.cuh"
 #include "sr_traverse.cuh"
 #include "sr_fan.cuh"
@@ -1056,7 +1057,8 @@ __global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchAr
         const FanTile t = fan_tile(a, tile);
         const bool pair = part >= FAN_GROUPS;
         if (pair) part -= FAN_GROUPS;
-        const FanParts g = fan_parts(tw_log, th_log, whole ? tw_log + th_log : (pair ? FAN_PAIR_LOG : FAN_GROUP_LOG));
+        const uint32_t size_log = whole ? tw_log + th_log : (pair ? FAN_PAIR_LOG : FAN_GROUP_LOG);
+        const FanParts g = fan_parts(tw_log, th_log, size_log);
         const uint32_t x0 = part_x(g, part), y0 = part_y(g, part);  // in the tile
         uint32_t casts;
         const bool done = fan_pixels<OCT>(a, t.obs, t.x + x0, t.y + y0, g.w_log, g.h_log, !whole, pair ? FAN_UNLIMITED : FAN_BUDGET,
@@ -1068,8 +1070,8 @@ __global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchAr
             const uint32_t px = x0 + ((2u * lane) & ((1u << g.w_log) - 1u)), py = y0 + ((2u * lane) >> g.w_log);
             if (pair) {
                 if (lane == 0) atomicOr(a.err, ERR_TRAVERSAL_LIMIT);
-            } else if (whole) {
-                fan_push(q, tile, lane, lane < FAN_GROUPS);
+            } else if (size_log > FAN_GROUP_LOG) {
+                fan_push(q, tile, lane, lane < (1u << (size_log - FAN_GROUP_LOG)));
             } else {
                 fan_push(q, tile, FAN_GROUPS + ((py >> p.h_log) << p.across) + (px >> p.w_log), lane < (1u << (FAN_GROUP_LOG - FAN_PAIR_LOG)));
             }
@@ -1098,7 +1100,8 @@ __global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ Trac
         const FanParts g = fan_parts(tw_log, th_log, half ? tw_log + th_log : (pair ? FAN_PAIR_LOG : FAN_GROUP_LOG));
         const uint32_t k = half ? 0u : part - FAN_HALVES - (pair ? FAN_GROUPS : 0u);
         const FanTile t = fan_tile(a, tile);
-        const uint32_t i = half ? 32u * part + lane : lane, n = half ? 64u : 1u << (g.w_log + g.h_log);
+        const uint32_t n = 1u << (g.w_log + g.h_log - (half ? 1u : 0u));  // the task's pixels
+        const uint32_t i = (half ? n * part : 0u) + lane;
         const uint32_t x = part_x(g, k) + (i & ((1u << g.w_log) - 1u)), y = part_y(g, k) + (i >> g.w_log);  // in the tile
         const ObsDev& od = a.obs[t.obs];
         const uint32_t px = t.x + x, py = t.y + y, pix = od.pix_base + py * od.width + px;
@@ -1107,7 +1110,7 @@ __global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ Trac
         s.d = v4(0.0f, 0.0f, 1.0f, 0.0f);
         s.t_max = 0.0f;
         s.enters = false;
-        const bool query = i < n && px < od.width && py < od.height &&
+        const bool query = lane < n && px < od.width && py < od.height &&
                            fan_query(a, t.obs, px, py, pix, &s);
         const bool enters = query && s.enters;
         bool hit = false, done = true;
@@ -1357,6 +1360,179 @@ Shape make_shape(const BatchRequest& r, uint32_t tile_w, uint32_t tile_h) {
 
 }  // namespace
 
+static WideScene wide_scene(const FastScene& s, const SceneDev& sd) {
+    WideScene ws;
+    ws.boxes = s.boxes.as<float4>();
+    ws.oct_stride = 4ull * s.num_wide;
+    ws.refs = s.refs.as<uint2>();
+    ws.up = s.up.as<uint32_t>();
+    ws.leafpar = s.leafpar.as<uint32_t>();
+    ws.geoms = sd.geoms;
+    ws.root_min = make_float4(s.root_min[0], s.root_min[1], s.root_min[2], s.root_min[3]);
+    ws.root_max = make_float4(s.root_max[0], s.root_max[1], s.root_max[2], s.root_max[3]);
+    ws.root_ref = s.root_ref;
+    ws.empty = s.empty ? 1u : 0u;
+    ws.fan_box = s.fan_box.as<float4>();
+    ws.fan_ref = s.fan_ref.as<uint32_t>();
+    ws.fan_root = s.fan_root;
+    ws.leaf_bits = 0;
+    while (s.max_leaf >> ws.leaf_bits) ++ws.leaf_bits;
+    ws.oct_copies = s.copies == 16 ? 1u : 0u;
+    return ws;
+}
+
+// Whether the node layouts give a ray trace_ref's hit bit for bit: their comparisons assume a positive range
+// and finite values (no product of a coordinate, an inverse direction and a box overflows to a NaN).
+__device__ __forceinline__ bool layout_ray(float4 o, float4 d, float t_min, float t_max) {
+    const float lim = 1e12f;
+    const auto in = [&](float v) { return fabsf(v) <= lim; };  // false for a NaN
+    return t_min > 0.0f && t_max > 0.0f && in(o.x) && in(o.y) && in(o.z) && in(o.w) && in(d.x) && in(d.y) && in(d.z) && in(d.w);
+}
+
+__device__ __forceinline__ void write_ray_hit(const SceneDev& s, double a0, double a1, double a2, double a3, float4 o, float4 d,
+                                              int slot, const GeomHit& gh, SrRayHit* to) {
+    SrRayHit out;
+    out.id = 0xFFFFFFFFu;
+    out.slot = 0xFFFFFFFFu;
+    out.lambda = out.proper_time = 0.0f;
+    for (int k = 0; k < 4; ++k) { out.event[k] = 0.0; out.tet_bary[k] = 0.0f; }
+    out.uv[0] = out.uv[1] = 0.0f;
+    out.material = out.pad = 0u;
+    if (slot >= 0) {
+        Hit h;
+        interpolate(s.attrs + 12u * (uint32_t)slot, o, d, gh, &h);
+        out.slot = (uint32_t)slot;
+        out.id = s.leaf_to_orig ? __ldg(s.leaf_to_orig + slot) : (uint32_t)slot;
+        out.lambda = h.lambda;
+        out.proper_time = h.tau;
+        out.event[0] = (double)h.event.x + a0;
+        out.event[1] = (double)h.event.y + a1;
+        out.event[2] = (double)h.event.z + a2;
+        out.event[3] = (double)h.event.w + a3;
+        out.tet_bary[0] = h.b0;
+        out.tet_bary[1] = h.b1;
+        out.tet_bary[2] = h.b2;
+        out.tet_bary[3] = h.b3;
+        out.uv[0] = h.uv_u;
+        out.uv[1] = h.uv_v;
+        out.material = h.material;
+    }
+    *to = out;
+}
+
+// Caller rays (sr_trace_rays), one thread per ray on the reference's nodes: scenes without the layouts.
+__global__ void __launch_bounds__(64) k_trace_rays(const SceneDev s, double a0, double a1, double a2, double a3, const SrRay* rays,
+                                                   uint32_t n, SrRayHit* hits, uint32_t* counters) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const SrRay r = rays[i];
+    const float4 o = v4((float)(r.origin[0] - a0), (float)(r.origin[1] - a1), (float)(r.origin[2] - a2),
+                        (float)(r.origin[3] - a3));
+    const float4 d = v4(r.dir[0], r.dir[1], r.dir[2], r.dir[3]);
+    GeomHit gh{0.0f, 0.0f, 0.0f, 0.0f};
+    const int slot = trace_ref(s, o, d, r.t_min, r.t_max, &gh, counters + 1);
+    write_ray_hit(s, a0, a1, a2, a3, o, d, slot, gh, hits + i);
+}
+
+// Caller rays on the fan layout, one warp per ray: boxes and records one per lane against the ray itself,
+// nearest subtree first. A ray's own walk over binary nodes, one thread per ray, is a chain of dependent
+// loads, and the call waits for its longest: 4096 rays into 1M tetrahedra took 670 us.
+//
+// The hit is the reference's. Of the records that the ray hits and whose leaf box it enters, let k have the
+// smallest lambda; when the box's entry parameter as computed is not beyond it, every box on the way to
+// k is entered before any hit so far (boxes hold their children's), so the reference tests k, and no
+// nearer one. A hit before its box's entry is rounding against the build's padding; boxes are culled only
+// 0.1% beyond the closest hit, so that one is met rather than culled, and the ray then takes the
+// reference's own walk. Of hits at equal lambda the reference keeps the one its order meets first
+// (packet_precedes).
+template <bool OCT>
+__global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const __grid_constant__ WideScene ws, double a0, double a1,
+                                                        double a2, double a3, const SrRay* rays, uint32_t n, SrRayHit* hits,
+                                                        uint32_t* counters) {
+    const uint32_t i = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (i >= n) return;
+    const SrRay r = rays[i];
+    const float4 o = v4((float)(r.origin[0] - a0), (float)(r.origin[1] - a1), (float)(r.origin[2] - a2),
+                        (float)(r.origin[3] - a3));
+    const float4 d = v4(r.dir[0], r.dir[1], r.dir[2], r.dir[3]);
+    const float4 no = neg4(o), inv = v4(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z), safe_inv(d.w));
+    GeomHit best{0.0f, 0.0f, 0.0f, 0.0f};
+    int slot = -1;
+    bool reference = !layout_ray(o, d, r.t_min, r.t_max);
+    float en, ex;
+    slab_interval(ws.root_min, ws.root_max, no, inv, r.t_min, r.t_max, &en, &ex);
+    if (!reference && !ws.empty && ex >= en && en < r.t_max) {
+        uint2 st[FAN_LEVELS];
+        float t_max = r.t_max, limit = t_max;  // limit: boxes entered beyond it are culled
+        uint32_t node = ws.fan_root, depth = 0, visits = 0;
+        for (;;) {
+            if (++visits > MAX_VISITS_FAST) {
+                if (lane == 0) atomicOr(counters + 1, ERR_TRAVERSAL_LIMIT);
+                break;
+            }
+            const float4* bx = ws.fan_box + (size_t)node * 64u;
+            uint32_t ref = __ldg(ws.fan_ref + (size_t)node * 32u + lane);
+            slab_interval(__ldg(bx + lane), __ldg(bx + 32u + lane), no, inv, r.t_min, limit, &en, &ex);
+            const bool meets = ex >= en, leaf = (ref & REF_LEAF) != 0u;
+            uint32_t key = meets && !leaf ? ((__float_as_uint(en) & ~31u) | lane) : FAN_NONE;
+            FanDeal deal{__ballot_sync(FULL_WARP, meets && leaf), 0u, 0u, 0u};
+            while (deal.leaves | deal.left) {
+                uint32_t mine, from;
+                const uint32_t held = fan_deal(deal, ref, lane, mine, from);
+                const float entry = __shfl_sync(FULL_WARP, en, from);
+                GeomHit gh;
+                // Hits up to and including t_max, so that a hit at the closest hit's lambda is seen.
+                const bool h = lane < held && intersect_lean(ws.geoms + 5u * mine, no, d, r.t_min,
+                                                             __uint_as_float(__float_as_uint(t_max) + 1u), &gh);
+                if (!__any_sync(FULL_WARP, h)) continue;
+                if (__any_sync(FULL_WARP, h && gh.lambda < entry)) reference = true;
+                const uint32_t nearest = redux_min(h ? __float_as_uint(gh.lambda) : FAN_NONE);
+                for (uint32_t m = __ballot_sync(FULL_WARP, h && __float_as_uint(gh.lambda) == nearest); m; m &= m - 1u) {
+                    const uint32_t c = (uint32_t)__ffs((int)m) - 1u, rec = __shfl_sync(FULL_WARP, mine, c);
+                    const GeomHit g{__shfl_sync(FULL_WARP, gh.lambda, c), __shfl_sync(FULL_WARP, gh.u, c),
+                                    __shfl_sync(FULL_WARP, gh.v, c), __shfl_sync(FULL_WARP, gh.w, c)};
+                    if (g.lambda < t_max ||
+                        (slot >= 0 && packet_precedes<OCT>(ws, rec, (uint32_t)slot, no, inv, r.t_min, counters + 1))) {
+                        t_max = g.lambda;
+                        best = g;
+                        slot = (int)rec;
+                    }
+                }
+                limit = fminf(r.t_max, t_max * 1.001f);
+            }
+            uint32_t k = redux_min(key);
+            while ((k & ~31u) > __float_as_uint(limit) && depth > 0) {
+                const uint2 e = st[--depth];
+                key = e.x;
+                ref = e.y;
+                k = redux_min(key);
+            }
+            if ((k & ~31u) > __float_as_uint(limit)) break;
+            const uint32_t c = k & 31u;
+            node = __shfl_sync(FULL_WARP, ref, c);
+            if (lane == c) key = FAN_NONE;
+            st[depth++] = make_uint2(key, ref);
+        }
+    }
+    if (reference) slot = trace_ref(s, o, d, r.t_min, r.t_max, &best, counters + 1);  // the same for every lane
+    if (lane == 0) write_ray_hit(s, a0, a1, a2, a3, o, d, slot, best, hits + i);
+}
+
+cudaError_t fast_trace_rays(const FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
+                            SrRayHit* hits, uint32_t* counters, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    const WideScene ws = wide_scene(s, sd);
+    const double *a = anchor;
+    const uint32_t blocks = (n + 3) / 4;
+    if (!s.usable || s.fan_levels == 0)
+        k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, hits, counters);
+    else if (ws.oct_copies)
+        k_trace_rays_fan<true><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, hits, counters);
+    else
+        k_trace_rays_fan<false><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, hits, counters);
+    return cudaGetLastError();
+}
+
 float4* fast_batch_hdr(FastCtx& c, uint32_t pyr_base) { return c.hdr.as<float4>() + pyr_base; }
 
 cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd,
@@ -1368,8 +1544,12 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     bool packet = t.packet != 0 && !r.count_work && (s.empty || s.fan_levels != 0);
     Shape sh;
     uint32_t tile_w = t.tile_w, tile_h = t.tile_h;
-    if (packet) {  // 64-pixel tiles: the shorter side doubled
+    if (packet) {
+        uint64_t pixels = 0;
+        for (uint32_t i = 0; i < r.n; ++i) pixels += (uint64_t)r.u[i].size[0] * r.u[i].size[1];
+        const uint32_t size_log = getenv("FAN_T") ? atoi(getenv("FAN_T")) : 6;
         (tile_w < tile_h ? tile_w : tile_h) *= 2;
+        while (tile_w * tile_h > (1u << size_log)) (tile_w > tile_h ? tile_w : tile_h) /= 2;
         sh = make_shape(r, tile_w, tile_h);
         const size_t old = c.fan_list.bytes, old_shadows = c.fan_shadows.bytes;
         // Without room for the queue the rays walk alone. The queue's own buffer: its entries are zero
@@ -1453,22 +1633,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     std::memcpy(c.hlvl.p, sh.pre.data(), sh.pre.size() * 4);
 
     uint32_t* rgb = r.rgb ? r.rgb : c.rgb.as<uint32_t>();
-    WideScene ws;
-    ws.boxes = s.boxes.as<float4>();
-    ws.oct_stride = 4ull * s.num_wide;
-    ws.refs = s.refs.as<uint2>();
-    ws.up = s.up.as<uint32_t>();
-    ws.leafpar = s.leafpar.as<uint32_t>();
-    ws.geoms = sd.geoms;
-    ws.root_min = make_float4(s.root_min[0], s.root_min[1], s.root_min[2], s.root_min[3]);
-    ws.root_max = make_float4(s.root_max[0], s.root_max[1], s.root_max[2], s.root_max[3]);
-    ws.root_ref = s.root_ref;
-    ws.empty = s.empty ? 1u : 0u;
-    ws.fan_box = s.fan_box.as<float4>();
-    ws.fan_ref = s.fan_ref.as<uint32_t>();
-    ws.fan_root = s.fan_root;
-    ws.leaf_bits = 0;
-    while (s.max_leaf >> ws.leaf_bits) ++ws.leaf_bits;
+    const WideScene ws = wide_scene(s, sd);
     unsigned long long* work = reinterpret_cast<unsigned long long*>(counters + 4);
     const uint32_t* tile_pre = c.lvl_pre.as<uint32_t>();
     const uint32_t* pix_pre = tile_pre + stride;

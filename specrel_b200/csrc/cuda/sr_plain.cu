@@ -3,84 +3,12 @@
 // shading, shadow rays and the star term. It is the baseline the fast path is measured against,
 // and it reproduces the reference traversal order exactly (ties at equal lambda included).
 #include "sr_kernels.h"
+#include "sr_ref.cuh"
 #include "sr_shade.cuh"
 
 namespace srk {
 
 using namespace srd;
-
-// Iteration bound per ray: a tree checked at upload never gets near it; a corrupted one sets
-// ERR_TRAVERSAL_LIMIT and the ray ends instead of spinning.
-constexpr uint32_t MAX_VISITS = 1u << 22;
-
-struct NodeRef {
-    float4 bmin, bmax;
-    uint4 meta;  // right_or_first, count, left, pad
-};
-__device__ __forceinline__ NodeRef load_node(const SrGpuNode* nodes, uint32_t i) {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    NodeRef n;
-    n.bmin = __ldg(p);
-    n.bmax = __ldg(p + 1);
-    n.meta = __ldg(reinterpret_cast<const uint4*>(p + 2));
-    return n;
-}
-__device__ __forceinline__ float child_enter(const SrGpuNode* nodes, uint32_t i, float4 o, float4 inv, float t_min,
-                                             float t_max) {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    return slab_enter(__ldg(p), __ldg(p + 1), o, inv, t_min, t_max);
-}
-
-// Bvh4D::trace (bvh4d.rs:445-520). Returns the leaf slot of the closest hit or -1.
-__device__ int trace_ref(const SceneDev& s, float4 o, float4 d, float t_min, float t_max, GeomHit* best,
-                         uint32_t* err) {
-    if (s.num_nodes == 0u) return -1;
-    float4 inv = v4(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z), safe_inv(d.w));
-    float re = child_enter(s.nodes, 0, o, inv, t_min, t_max);
-    if (re < 0.0f) return -1;
-    uint32_t sn[SR_STACK_SIZE];
-    float stt[SR_STACK_SIZE];
-    uint32_t sp = 1;
-    sn[0] = 0;
-    stt[0] = re;
-    int slot = -1;
-    uint32_t visits = 0;
-    while (sp > 0) {
-        if (++visits > MAX_VISITS) { atomicOr(err, ERR_TRAVERSAL_LIMIT); break; }
-        --sp;
-        uint32_t ni = sn[sp];
-        if (stt[sp] >= t_max) continue;
-        uint4 meta = __ldg(reinterpret_cast<const uint4*>(s.nodes + ni) + 2);
-        if (meta.y > 0u) {
-            uint32_t first = meta.x, end = meta.x + meta.y;
-            for (uint32_t k = first; k < end; ++k) {
-                GeomHit gh;
-                if (intersect_geom(s.geoms + 5u * k, o, d, t_min, t_max, &gh)) {
-                    t_max = gh.lambda;
-                    *best = gh;
-                    slot = (int)k;
-                }
-            }
-        } else {
-            uint32_t li = meta.z, ri = meta.x;
-            float tl = child_enter(s.nodes, li, o, inv, t_min, t_max);
-            float tr = child_enter(s.nodes, ri, o, inv, t_min, t_max);
-            bool hl = tl >= 0.0f, hr = tr >= 0.0f;
-            if (hl && hr) {
-                if (sp + 2u <= SR_STACK_SIZE) {
-                    if (tl <= tr) { sn[sp] = ri; stt[sp] = tr; sn[sp + 1] = li; stt[sp + 1] = tl; }
-                    else { sn[sp] = li; stt[sp] = tl; sn[sp + 1] = ri; stt[sp + 1] = tr; }
-                    sp += 2u;
-                }
-            } else if (hl) {
-                if (sp < SR_STACK_SIZE) { sn[sp] = li; stt[sp] = tl; ++sp; }
-            } else if (hr) {
-                if (sp < SR_STACK_SIZE) { sn[sp] = ri; stt[sp] = tr; ++sp; }
-            }
-        }
-    }
-    return slot;
-}
 
 // Bvh4D::is_occluded (bvh4d.rs:523-578).
 __device__ bool occluded_ref(const SceneDev& s, float4 o, float4 d, float t_min, float t_max, uint32_t* err) {
@@ -154,54 +82,6 @@ cudaError_t launch_render_plain(const SceneDev& s, const SrGpuUniforms& u, const
     dim3 block(8, 8);
     dim3 grid((u.size[0] + 7) / 8, (u.size[1] + 7) / 8);
     k_render_plain<<<grid, block, 0, st>>>(s, u, cam_dev, f, bb);
-    return cudaGetLastError();
-}
-
-// Caller rays (sr_trace_rays): one thread per ray, the reference's traversal, then the hit
-// record interpolated as the shading reads it.
-__global__ void k_trace_rays(SceneDev s, double a0, double a1, double a2, double a3, const SrRay* rays, uint32_t n,
-                             SrRayHit* hits, uint32_t* counters) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const SrRay r = rays[i];
-    const float4 o = v4((float)(r.origin[0] - a0), (float)(r.origin[1] - a1), (float)(r.origin[2] - a2),
-                        (float)(r.origin[3] - a3));
-    const float4 d = v4(r.dir[0], r.dir[1], r.dir[2], r.dir[3]);
-    SrRayHit out;
-    out.id = 0xFFFFFFFFu;
-    out.slot = 0xFFFFFFFFu;
-    out.lambda = out.proper_time = 0.0f;
-    for (int k = 0; k < 4; ++k) { out.event[k] = 0.0; out.tet_bary[k] = 0.0f; }
-    out.uv[0] = out.uv[1] = 0.0f;
-    out.material = out.pad = 0u;
-    GeomHit gh;
-    const int slot = trace_ref(s, o, d, r.t_min, r.t_max, &gh, counters + 1);
-    if (slot >= 0) {
-        Hit h;
-        interpolate(s.attrs + 12u * (uint32_t)slot, o, d, gh, &h);
-        out.slot = (uint32_t)slot;
-        out.id = s.leaf_to_orig ? __ldg(s.leaf_to_orig + slot) : (uint32_t)slot;
-        out.lambda = h.lambda;
-        out.proper_time = h.tau;
-        out.event[0] = (double)h.event.x + a0;
-        out.event[1] = (double)h.event.y + a1;
-        out.event[2] = (double)h.event.z + a2;
-        out.event[3] = (double)h.event.w + a3;
-        out.tet_bary[0] = h.b0;
-        out.tet_bary[1] = h.b1;
-        out.tet_bary[2] = h.b2;
-        out.tet_bary[3] = h.b3;
-        out.uv[0] = h.uv_u;
-        out.uv[1] = h.uv_v;
-        out.material = h.material;
-    }
-    hits[i] = out;
-}
-
-cudaError_t launch_trace_rays(const SceneDev& s, const double anchor[4], const SrRay* rays, uint32_t n, SrRayHit* hits,
-                              uint32_t* counters, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    k_trace_rays<<<(n + 127) / 128, 128, 0, st>>>(s, anchor[0], anchor[1], anchor[2], anchor[3], rays, n, hits, counters);
     return cudaGetLastError();
 }
 

@@ -68,6 +68,7 @@ struct WideScene {
     const uint32_t* fan_ref;
     uint32_t fan_root;
     uint32_t leaf_bits;  // bits of the largest leaf's primitive count
+    uint32_t oct_copies; // the 16 octant copies are there (else one)
 };
 
 // Traversal work of one thread (the SR_FLAG_COUNT_WORK variant only).

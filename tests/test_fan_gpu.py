@@ -116,3 +116,34 @@ def test_frames_of_growing_size_in_turn(engine, bodies):
     for w, h in ((96, 64), (320, 200), (200, 120), (640, 400), (96, 64), (800, 500)):
         u, cam = _u(bodies, w, h, (-0.9, 0.8, 1.0))
         _both(engine, IDX, u, cam)
+
+
+@pytest.mark.parametrize("layout", [L.SR_LAYOUT_OCTANT, L.SR_LAYOUT_COMPACT])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 3000])
+def test_caller_rays_on_the_node_layout(engine, bodies, layout, n):
+    """sr_trace_rays walks the node layout for rays of a positive finite range and the reference's nodes for
+    others: a ray cast alone, among others and in another block position has the same hit, and rays of
+    odd ranges (zero, negative, endless) the hits of the same rays within that range."""
+    engine.set_layout(IDX, layout)
+    try:
+        rng = np.random.default_rng(n)
+        d = rng.normal(size=(n, 3))
+        rays = np.zeros((n, 10))
+        rays[:, 4], rays[:, 5:8] = -1.0, d / np.linalg.norm(d, axis=1, keepdims=True)
+        rays[:, 8], rays[:, 9] = 1e-3, 180.0
+        h = engine.trace_rays(IDX, rays)
+        back = engine.trace_rays(IDX, rays[::-1])[::-1]
+        assert h.tobytes() == back.tobytes()
+        odd = rays.copy()
+        odd[:, 8] = 0.0  # the reference's nodes: no geometry lies at the observer, so the same hits
+        o = engine.trace_rays(IDX, odd)
+        near = (o["lambda_"] != h["lambda_"]) & (o["lambda_"] < 1e-3)
+        assert (o["slot"][~near] == h["slot"][~near]).all() and (o["lambda_"][~near] == h["lambda_"][~near]).all()
+        odd[:, 8], odd[:, 9] = 1e-3, np.inf
+        e = engine.trace_rays(IDX, odd)
+        hit = h["slot"] != 0xFFFFFFFF
+        assert (e["slot"][hit] == h["slot"][hit]).all()
+        with pytest.raises(ValueError):
+            engine.trace_rays(IDX, np.zeros((2, 1)))
+    finally:
+        engine.set_layout(IDX, L.SR_LAYOUT_AUTO)
