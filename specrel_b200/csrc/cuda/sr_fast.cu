@@ -35,28 +35,45 @@ using namespace srd;
 // Layout build.
 // ---------------------------------------------------------------------------------------------
 // The internal nodes of the top TOP_LEVELS levels, breadth first, from an internal root (node 0):
-// topid[node] = its position + 1 (topid zeroed before), level_end[k] = nodes in levels 0..k. One
-// thread: at most TOP_NODES nodes, once per layout build.
-__global__ void k_top_levels(const SrGpuNode* nodes, uint32_t* topid, uint32_t* level_end) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    uint32_t q[TOP_NODES];
-    uint32_t m = 1, start = 0, end = 1;
-    q[0] = 0;
-    topid[0] = 1;
-    level_end[0] = 1;
+// topid[node] = its position + 1 (topid zeroed before), level_end[k] = nodes in levels 0..k. One block, a
+// node of the level per thread (one thread for all of them took 94 us, 2% of a small rebuild).
+__global__ void __launch_bounds__(TOP_NODES / 2 + 1) k_top_levels(const SrGpuNode* nodes, uint32_t* topid, uint32_t* level_end) {
+    __shared__ uint32_t q[TOP_NODES], per_warp[(TOP_NODES / 2 + 1) / 32];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    uint32_t start = 0, end = 1;
+    if (t == 0) {
+        q[0] = 0;
+        topid[0] = 1;
+        level_end[0] = 1;
+    }
+    __syncthreads();
     for (uint32_t lv = 1; lv < TOP_LEVELS; ++lv) {
-        for (uint32_t i = start; i < end; ++i) {
-            const SrGpuNode& nd = nodes[q[i]];
-            const uint32_t c[2] = {nd.left, nd.right_or_first};
-            for (int k = 0; k < 2; ++k)
-                if (nodes[c[k]].count == 0 && m < TOP_NODES) {
-                    q[m] = c[k];
-                    topid[c[k]] = ++m;
-                }
+        uint32_t c[2] = {0, 0};
+        bool in[2] = {false, false};
+        if (start + t < end) {
+            const SrGpuNode& nd = nodes[q[start + t]];
+            c[0] = nd.left;
+            c[1] = nd.right_or_first;
+            for (int k = 0; k < 2; ++k) in[k] = nodes[c[k]].count == 0;
         }
+        const uint32_t ml = __ballot_sync(0xFFFFFFFFu, in[0]), mr = __ballot_sync(0xFFFFFFFFu, in[1]);
+        if (lane == 0) per_warp[warp] = (uint32_t)(__popc(ml) + __popc(mr));
+        __syncthreads();
+        const uint32_t below = (1u << lane) - 1u;
+        uint32_t at = end + (uint32_t)(__popc(ml & below) + __popc(mr & below)), total = 0;
+        for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
+            if (w < warp) at += per_warp[w];
+            total += per_warp[w];
+        }
+        for (int k = 0; k < 2; ++k)
+            if (in[k]) {
+                q[at] = c[k];
+                topid[c[k]] = ++at;
+            }
         start = end;
-        end = m;
-        level_end[lv] = m;
+        end += total;
+        if (t == 0) level_end[lv] = end;
+        __syncthreads();
     }
 }
 
@@ -108,6 +125,7 @@ __global__ void k_wide_fill(const SrGpuNode* nodes, uint32_t n, const uint32_t* 
 }
 
 static cudaError_t lean_kernel_attrs(int max_smem);
+static cudaError_t fan_resident(int threads, int* blocks);
 bool lean_stack_supported(uint32_t s);
 
 // Dynamic shared memory of the lean kernel: S + 1 stack words per thread (S of them used).
@@ -118,6 +136,13 @@ static size_t lean_stack_bytes(const SrTuning& t) {
 cudaError_t fast_init(FastCtx& c, const cudaDeviceProp& prop) {
     c.num_sms = prop.multiProcessorCount;
     c.max_smem = (int)prop.sharedMemPerBlockOptin;
+    const int sizes[4] = {64, 128, 256, 512};
+    for (int threads : sizes) {
+        int n = 0;
+        cudaError_t e = fan_resident(threads, &n);
+        if (e != cudaSuccess) return e;
+        c.fan_blocks[threads / 128] = (uint32_t)std::max(n, 1);
+    }
     return lean_kernel_attrs(c.max_smem);
 }
 
@@ -169,7 +194,7 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
     uintptr_t tp = reinterpret_cast<uintptr_t>(level_end + 16);
     void* tmp = reinterpret_cast<void*>((tp + 255) & ~uintptr_t(255));
     if ((e = cudaMemsetAsync(topid, 0, (size_t)n * 4 + 64, st)) != cudaSuccess) return e;
-    k_top_levels<<<1, 1, 0, st>>>(nodes, topid, level_end);
+    k_top_levels<<<1, TOP_NODES / 2 + 1, 0, st>>>(nodes, topid, level_end);
     k_wide_flags<<<(n + 255) / 256, 256, 0, st>>>(nodes, n, topid, flags);
     if ((e = cub::DeviceScan::ExclusiveSum(tmp, temp, flags, wid, (int)n, st)) != cudaSuccess) return e;
     uint32_t last[2] = {0, 0};
@@ -818,6 +843,9 @@ struct FanTasks {
     uint32_t waste;     // FAN_WASTE or FAN_WASTE_SMALL
 };
 
+// log2 of a tile's pixels: 64, fewer where that leaves less than a tile or so per warp.
+static uint32_t fan_tile_log(uint64_t pixels) { return pixels < (128u << 10) ? 3u : (pixels < (512u << 10) ? 4u : 6u); }
+
 __device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -888,7 +916,7 @@ __device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, 
                     const uint32_t tail = load_acquire(q.count + FAN_TAIL);
                     if (finished == tail && tail <= ticket) break;
                 }
-                __nanosleep(1000);
+                __nanosleep(200);
             }
             if (polls > FAN_POLLS) {
                 atomicOr(err, ERR_BAD_INDEX);
@@ -1037,12 +1065,14 @@ __global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchAr
     uint2 st[FAN_LEVELS];
     const uint32_t tiles = a.total_rays >> 5, tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t mine = 0;
+    uint32_t mine = 0, ahead = 0;  // ahead: the next tile, asked for a tile early (lane 0)
+    if (lane == 0) ahead = atomicAdd(q.count + FAN_NEXT, 1u);
     bool whole = true;  // whole tiles first, then the queue
     for (;;) {
         uint32_t tile, part = 0;
         if (whole) {
-            tile = warp_next(q.count + FAN_NEXT);
+            tile = __shfl_sync(FULL_WARP, ahead, 0);
+            if (lane == 0 && tile < tiles) ahead = atomicAdd(q.count + FAN_NEXT, 1u);
             if (tile >= tiles) {
                 fan_first_done(q, mine);
                 whole = false;
@@ -1137,6 +1167,11 @@ __global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ Trac
         }
         fan_finished(q);
     }
+}
+
+// Resident blocks per SM of k_fan_trace.
+static cudaError_t fan_resident(int threads, int* blocks) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_fan_trace<true>, threads, (size_t)(threads / 32) * sizeof(FanQueue));
 }
 
 // The shared-memory stack depths the lean kernel is built for (SrTuning.stack_smem).
@@ -1547,7 +1582,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     if (packet) {
         uint64_t pixels = 0;
         for (uint32_t i = 0; i < r.n; ++i) pixels += (uint64_t)r.u[i].size[0] * r.u[i].size[1];
-        const uint32_t size_log = getenv("FAN_T") ? atoi(getenv("FAN_T")) : 6;
+        const uint32_t size_log = getenv("FAN_T") ? atoi(getenv("FAN_T")) : fan_tile_log(pixels);
         (tile_w < tile_h ? tile_w : tile_h) *= 2;
         while (tile_w * tile_h > (1u << size_log)) (tile_w > tile_h ? tile_w : tile_h) /= 2;
         sh = make_shape(r, tile_w, tile_h);
@@ -1677,7 +1712,9 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         ta.work = work;
         uint32_t blocks = (uint32_t)c.num_sms * t.blocks_per_sm;
         uint32_t need = (uint32_t)(((uint64_t)sh.total_tiles * 32 + t.block_threads - 1) / t.block_threads);
-        if (packet) need = blocks;  // a small frame's slow tiles are split among the warps that have none
+        // Blocks beyond the resident ones would start when the work is done; a small frame's slow tiles are
+        // split among the warps that have none.
+        if (packet) need = (uint32_t)c.num_sms * c.fan_blocks[t.block_threads / 128u];
         if (blocks > need) blocks = need;
         const size_t smem = t.leaf_coop ? (size_t)(t.block_threads / 32) * COOP_SMEM_PER_WARP : 0;
         const bool lean = !t.leaf_coop && t.leaf_batch == 1 && t.refill_lanes == 32 && t.chunk_tiles == 1;

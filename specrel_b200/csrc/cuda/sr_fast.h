@@ -97,6 +97,7 @@ struct GraphEntry {
 struct FastCtx {
     int num_sms = 148;
     int max_smem = 0;
+    uint32_t fan_blocks[5] = {1, 1, 1, 1, 1};  // resident blocks per SM of k_fan_trace, by threads / 128
     // Batch buffers, grown on demand.
     // shadow: one byte per pixel, the main light's shadow ray as traced (0 none, 1 clear, 2 occluded)
     // sched: the tile counters of the trace kernel, one per SM band then the shared pool's
