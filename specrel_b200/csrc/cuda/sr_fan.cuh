@@ -29,7 +29,9 @@ constexpr int FAN_RAYS = 2;             // rays per lane of a closest-hit walk
 // five levels from the root leaves whatever remains there.
 // ---------------------------------------------------------------------------------------------
 struct FanCounts {
-    uint32_t units, fans, conflict, queue_end[FAST_MAX_DEPTH + 2];
+    uint32_t fans, conflict, root_total;
+    uint32_t units[FAN_LEVELS + 2];          // per level
+    uint32_t reached[FAST_MAX_DEPTH + 2];    // nodes per depth (the marking)
 };
 
 // parent[child] = i for both children of every internal node (of every reached node, when `reach` is
@@ -43,28 +45,24 @@ __global__ void k_fan_parents(const SrGpuNode* nodes, uint32_t n, const uint32_t
         if (c[k] >= n || c[k] == 0 || atomicExch(parent + c[k], i) != FAN_NONE) fc->conflict = 1;
 }
 
-// One level of the breadth-first marking: the nodes queue[queue_end[l - 1], queue_end[l]) put their
-// children behind them.
+// One level of the breadth-first marking: the nodes of depth `level`, which lie in the queue behind those of
+// the depths above, put their children behind them.
 __global__ void k_fan_reach(const SrGpuNode* nodes, uint32_t n, uint32_t* reach, uint32_t* queue, uint32_t level,
                             FanCounts* fc) {
-    const uint32_t begin = level ? fc->queue_end[level - 1] : 0u, end = fc->queue_end[level];
-    for (uint32_t q = begin + blockIdx.x * blockDim.x + threadIdx.x; q < end; q += gridDim.x * blockDim.x) {
-        const SrGpuNode& nd = nodes[queue[q]];
-        reach[queue[q]] = 1;
-        if (nd.count != 0) continue;
-        const uint32_t at = atomicAdd(&fc->queue_end[level + 1], 2u);
+    uint32_t begin = 0;
+    for (uint32_t l = 0; l < level; ++l) begin += fc->reached[l];
+    const uint32_t count = level ? fc->reached[level] : 1u;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        const uint32_t i = level ? queue[begin + q] : 0u;
+        if (level == 0) fc->reached[0] = 1;
+        reach[i] = 1;
+        if (nodes[i].count != 0) continue;
+        const uint32_t at = begin + count + atomicAdd(&fc->reached[level + 1], 2u);
         if (at + 1 < n) {
-            queue[at] = nd.left;
-            queue[at + 1] = nd.right_or_first;
+            queue[at] = nodes[i].left;
+            queue[at + 1] = nodes[i].right_or_first;
         }
     }
-}
-__global__ void k_fan_reach_begin(uint32_t* queue, uint32_t level, FanCounts* fc) {
-    if (level == 0) {
-        queue[0] = 0;
-        fc->queue_end[0] = 1;
-    }
-    fc->queue_end[level + 1] = fc->queue_end[level];
 }
 
 // Appends `v` to list[*count ...] for the lanes with `yes` (one atomic per warp); returns its place.
@@ -82,35 +80,38 @@ __global__ void k_fan_leaves(const SrGpuNode* nodes, uint32_t n, const uint32_t*
                              FanCounts* fc) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool leaf = i < n && nodes[i].count != 0 && (!reach || reach[i]);
-    fan_append(leaf, i, units, &fc->units);
+    fan_append(leaf, i, units, &fc->units[0]);
     if (leaf) uref[i] = pack_leaf(nodes[i].right_or_first, nodes[i].count);
 }
 
 // total[v] = the units below v where that is at most 32, else 0; acc: what the first child brought.
-__global__ void k_fan_climb(const uint32_t* units, uint32_t num_units, const uint32_t* parent, uint32_t* acc, uint32_t* total) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= num_units) return;
-    uint32_t v = units[i], c = 1;
-    total[v] = 1;
-    for (uint32_t up = 0; v != 0 && up <= FAST_MAX_DEPTH; ++up) {
-        const uint32_t p = parent[v];
-        if (p == FAN_NONE) return;
-        const uint32_t other = atomicAdd(acc + p, c);
-        if (other == 0) return;
-        c += other;
-        if (c > FAN) return;
-        total[p] = c;
-        v = p;
+__global__ void k_fan_climb(const uint32_t* units, uint32_t level, const uint32_t* parent, uint32_t* acc, uint32_t* total,
+                            const FanCounts* fc) {
+    const uint32_t num_units = fc->units[level];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < num_units; i += gridDim.x * blockDim.x) {
+        uint32_t v = units[i], c = 1;
+        total[v] = 1;
+        for (uint32_t up = 0; v != 0 && up <= FAST_MAX_DEPTH; ++up) {
+            const uint32_t p = parent[v];
+            if (p == FAN_NONE) break;
+            const uint32_t other = atomicAdd(acc + p, c);
+            if (other == 0) break;
+            c += other;
+            if (c > FAN) break;
+            total[p] = c;
+            v = p;
+        }
     }
 }
 
 // The units of the next level: the topmost counted nodes. Those of more than one unit become fan
 // nodes, numbered behind the ones of the levels below.
-__global__ void k_fan_units(uint32_t n, const uint32_t* parent, const uint32_t* total, uint32_t* uref, uint32_t* units,
-                            uint32_t* fan_root, FanCounts* fc) {
+__global__ void k_fan_units(uint32_t n, uint32_t level, const uint32_t* parent, const uint32_t* total, uint32_t* uref,
+                            uint32_t* units, uint32_t* fan_root, FanCounts* fc) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool unit = i < n && total[i] != 0 && (i == 0 || parent[i] == FAN_NONE || total[parent[i]] == 0);
-    fan_append(unit, i, units, &fc->units);
+    fan_append(unit, i, units, &fc->units[level + 1]);
+    if (i == 0) fc->root_total = total[0];
     const bool fan = unit && total[i] > 1;
     const uint32_t at = fan_append(fan, i, fan_root, &fc->fans);
     if (fan) uref[i] = at;
@@ -172,34 +173,30 @@ static cudaError_t fan_build(FastScene& s, const SrGpuNode* nodes, uint32_t n, u
     if ((e = look()) != cudaSuccess) return e;
     if (h.conflict) {
         if ((e = cudaMemsetAsync(parent, 0xFF, (size_t)n * 4, st)) != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(total, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(fc, 0, sizeof(FanCounts), st)) != cudaSuccess) return e;
-        uint32_t* mark = acc;  // cleared below before the counts use it; `total` is the queue
-        if ((e = cudaMemsetAsync(mark, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
-        for (uint32_t l = 0; l < s.depth && l < FAST_MAX_DEPTH; ++l) {
-            k_fan_reach_begin<<<1, 1, 0, st>>>(total, l, fc);
-            k_fan_reach<<<296, 128, 0, st>>>(nodes, n, mark, total, l, fc);
-        }
-        // The marks move to `roots`, which the fan numbering writes only after the leaves are listed.
-        if ((e = cudaMemcpyAsync(roots, mark, (size_t)n * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
+        // The marks lie in `roots`, which the fan numbering writes only after the leaves are listed; `total` is
+        // the queue.
+        if ((e = cudaMemsetAsync(roots, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
+        for (uint32_t l = 0; l < s.depth && l <= FAST_MAX_DEPTH; ++l)
+            k_fan_reach<<<148, 256, 0, st>>>(nodes, n, roots, total, l, fc);
         reach = roots;
         k_fan_parents<<<blocks, 256, 0, st>>>(nodes, n, reach, parent, fc);
-        if ((e = look()) != cudaSuccess) return e;
-        if (h.conflict) return cudaSuccess;  // not a tree: no fan layout
     }
     k_fan_leaves<<<blocks, 256, 0, st>>>(nodes, n, reach, uref, units, fc);
-    if ((e = look()) != cudaSuccess) return e;
-    uint32_t levels = 0, root_total = 0;
-    while (root_total == 0 && levels < FAN_LEVELS) {
+    // As many levels as a tree of this size usually has before the first look (each is a few launches, and a
+    // look waits for them), then one by one.
+    uint32_t levels = 0, usual = 1;
+    for (uint64_t k = n / 2; k > FAN; k /= 18) ++usual;
+    do {
         if ((e = cudaMemsetAsync(acc, 0, (size_t)n * 8, st)) != cudaSuccess) return e;  // acc and total
-        k_fan_climb<<<(h.units + 255) / 256, 256, 0, st>>>(units, h.units, parent, acc, total);
-        if ((e = cudaMemsetAsync(&fc->units, 0, 4, st)) != cudaSuccess) return e;
-        k_fan_units<<<blocks, 256, 0, st>>>(n, parent, total, uref, units, roots, fc);
-        if ((e = cudaMemcpyAsync(&root_total, total, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-        if ((e = look()) != cudaSuccess) return e;
+        k_fan_climb<<<std::min(blocks, 148u * 16u), 256, 0, st>>>(units, levels, parent, acc, total, fc);
+        k_fan_units<<<blocks, 256, 0, st>>>(n, levels, parent, total, uref, units, roots, fc);
         ++levels;
-    }
-    if (root_total == 0) return cudaSuccess;
+        if (levels < usual && levels < FAN_LEVELS) continue;
+        if ((e = look()) != cudaSuccess) return e;
+        if (h.conflict) return cudaSuccess;  // not a tree: no fan layout
+    } while (h.root_total == 0 && levels < FAN_LEVELS);
+    if (h.root_total == 0) return cudaSuccess;
     if (s.fan_box.ensure_grow((size_t)h.fans * 64 * sizeof(float4)) != cudaSuccess ||
         s.fan_ref.ensure_grow((size_t)h.fans * 32 * 4) != cudaSuccess) {
         cudaGetLastError();
