@@ -376,7 +376,7 @@ __global__ void k_large_events(const Chunk* chunks, const LTask* tasks, const ui
 // chains end within a few, and the rounds of pointer jumping that remain start from chains CHASE times
 // shorter.
 constexpr uint32_t CHASE_LOG = 8, CHASE = 1u << CHASE_LOG;
-__global__ void k_chase(const int* item_a, const int* ref_a, int* item_b, int* ref_b, uint32_t len) {
+__global__ void k_chase(const int* item_a, const int* ref_a, int* item_b, int* ref_b, uint32_t len, uint32_t* unresolved) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= len) return;
     int it = item_a[j], rf = ref_a[j];
@@ -386,12 +386,14 @@ __global__ void k_chase(const int* item_a, const int* ref_a, int* item_b, int* r
     }
     item_b[j] = it;
     ref_b[j] = rf;
+    if (it < 0 && rf >= 0) *unresolved = 1;
 }
 
-// One round of pointer jumping over the enqueue list (reads a, writes b).
-__global__ void k_jump(const int* item_a, const int* ref_a, int* item_b, int* ref_b, uint32_t len) {
+// One round of pointer jumping over the enqueue list (reads a, writes b); nothing where the chase resolved
+// every chain.
+__global__ void k_jump(const int* item_a, const int* ref_a, int* item_b, int* ref_b, uint32_t len, const uint32_t* unresolved) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= len) return;
+    if (j >= len || !*unresolved) return;
     int it = item_a[j], rf = ref_a[j];
     if (it < 0 && rf >= 0) {
         const int it2 = item_a[rf];
@@ -408,10 +410,12 @@ __global__ void k_jump(const int* item_a, const int* ref_a, int* item_b, int* re
 
 // The partitioned order: left elements at their left rank, then the queue's final contents.
 __global__ void k_large_scatter(const Chunk* chunks, const LTask* tasks, const LHead* heads, const uint32_t* perm,
-                                const uint32_t* flag, const uint32_t* lb, const int* eitem, uint32_t* perm_out) {
+                                const uint32_t* flag, const uint32_t* lb, const int* chased, const int* jumped,
+                                const uint32_t* unresolved, uint32_t* perm_out) {
     const Chunk c = chunks[blockIdx.x];
     const LTask t = tasks[c.task];
     const LHead& h = heads[c.task];
+    const int* eitem = *unresolved ? jumped : chased;
     for (uint32_t q = c.q0 + threadIdx.x; q < c.q1; q += blockDim.x) {
         const uint32_t i = q - t.qbase;
         if (h.leaf) {
@@ -642,6 +646,7 @@ struct TinyShared {
     int bl[32][4], bh[32][4];
     uint32_t bc[32];
     int red[16];
+    uint32_t lefts[TINY / 32];  // the elements of the node that go left, a bit each
     uint32_t fs[64], fc[64], fpatch[64], fdepth[64];
     uint32_t cur_s, cur_c, cur_patch, cur_depth;
     int sp, node_count, max_depth, max_leaf, bad;
@@ -765,20 +770,29 @@ __global__ void __launch_bounds__(32 * WARPS_TINY) k_small_build_warp(const STas
             __syncwarp();
         }
         const SplitChoice ch = decide_split_warp(w.red + 8, w.red + 12, w.bl, w.bh, w.bc, lane);
+        const bool split = !__shfl_sync(0xFFFFFFFFu, ch.leaf, 0);
+        if (split) {  // which elements go left, by lane
+            const int axis = __shfl_sync(0xFFFFFFFFu, ch.axis, 0);
+            const float pos = __shfl_sync(0xFFFFFFFFu, ch.pos, 0);
+            for (uint32_t i = 0; i < c; i += 32) {
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, i + lane < c && ax(w.cen[w.ord[s + min(i + lane, c - 1u)]], axis) < pos);
+                if (lane == 0) w.lefts[i >> 5] = m;
+            }
+            __syncwarp();
+        }
         if (lane == 0) {
-            int leaf = ch.leaf, axis = ch.axis;
-            const float pos = ch.pos;
+            int leaf = ch.leaf;
             uint32_t mid = 0;
             if (!leaf) {
-                // The reference's partition pass.
-                for (uint32_t i = 0; i < c; ++i) {
-                    const uint16_t e = w.ord[s + i];
-                    if (ax(w.cen[e], axis) < pos) {
+                // The reference's partition pass: it moves at the left elements only.
+                for (uint32_t k = 0; k < c; k += 32)
+                    for (uint32_t m = w.lefts[k >> 5]; m; m &= m - 1u) {
+                        const uint32_t i = k + (uint32_t)__ffs((int)m) - 1u;
+                        const uint16_t e = w.ord[s + i];
                         w.ord[s + i] = w.ord[s + mid];
                         w.ord[s + mid] = e;
                         ++mid;
                     }
-                }
                 if (mid == 0 || mid == c) {  // the reference selects by median here: not supported
                     w.bad = 1;
                     leaf = 1;
@@ -905,6 +919,7 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
     Buf<float4> cen;
     Buf<uint32_t> perm, perm2, flag, key, lb, svc, sb;
     Buf<int> ei[2], er[2];
+    Buf<uint32_t> unresolved;
     Buf<SrGpuNode> tmp;
     BK(cen.alloc(n, st));
     BK(perm.alloc(n, st));
@@ -955,6 +970,7 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
         cub::DeviceScan::ExclusiveSumByKey(nullptr, scan_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                            (uint32_t*)nullptr, (int)n);
         BK(scan_tmp.alloc(scan_bytes, st));
+        BK(unresolved.alloc(1, st));
         BK(flag.alloc(n, st));
         BK(key.alloc(n, st));
         BK(lb.alloc(n, st));
@@ -1006,14 +1022,15 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
         for (const LTask& tk : tasks) maxc = std::max(maxc, tk.count);
         int rounds = 1;
         while ((1ull << rounds) < 2ull * maxc + 2) ++rounds;
-        k_chase<<<(len + 255) / 256, 256, 0, st>>>(ei[cur].p, er[cur].p, ei[1 - cur].p, er[1 - cur].p, len);
+        BK(cudaMemsetAsync(unresolved.p, 0, 4, st));
+        k_chase<<<(len + 255) / 256, 256, 0, st>>>(ei[cur].p, er[cur].p, ei[1 - cur].p, er[1 - cur].p, len, unresolved.p);
         cur = 1 - cur;
         for (int round = (int)CHASE_LOG; round <= rounds; ++round) {
-            k_jump<<<(len + 255) / 256, 256, 0, st>>>(ei[cur].p, er[cur].p, ei[1 - cur].p, er[1 - cur].p, len);
+            k_jump<<<(len + 255) / 256, 256, 0, st>>>(ei[cur].p, er[cur].p, ei[1 - cur].p, er[1 - cur].p, len, unresolved.p);
             BK(cudaGetLastError());
             cur = 1 - cur;
         }
-        k_large_scatter<<<nch, 256, 0, st>>>(dc.p, dt.p, dh.p, perm.p, flag.p, lb.p, ei[cur].p, perm2.p);
+        k_large_scatter<<<nch, 256, 0, st>>>(dc.p, dt.p, dh.p, perm.p, flag.p, lb.p, ei[1].p, ei[cur].p, unresolved.p, perm2.p);
         k_copy_range<<<nch, 256, 0, st>>>(dc.p, dt.p, perm2.p, perm.p);
         BK(cudaGetLastError());
         std::vector<LHead> heads(nt);
