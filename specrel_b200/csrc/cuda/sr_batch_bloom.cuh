@@ -8,14 +8,9 @@ namespace srk {
 // level's pixel counts.
 __constant__ float DOWN_WB[4] = {0.125f, 0.375f, 0.375f, 0.125f};
 
-__global__ void k_bloom_down_batch(float4* hdr, const ObsDev* obs, const uint32_t* pre, uint32_t n, int k) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= __ldg(pre + n)) return;
-    uint32_t o = find_obs(pre, n, i);
-    const ObsDev& od = obs[o];
-    uint32_t l = i - __ldg(pre + o);
-    uint32_t dw = od.lw[k], x = l % dw, y = l / dw;
-    uint32_t sw = od.lw[k - 1], sh = od.lh[k - 1];
+// Pixel (x, y) of level k from level k - 1.
+__device__ __forceinline__ float4 bloom_down_px(const float4* hdr, const ObsDev& od, int k, uint32_t x, uint32_t y) {
+    const uint32_t sw = od.lw[k - 1], sh = od.lh[k - 1];
     const float4* src = hdr + od.pyr_base + od.loff[k - 1];
     float ax = 0.0f, ay = 0.0f, az = 0.0f;
 #pragma unroll
@@ -36,7 +31,16 @@ __global__ void k_bloom_down_batch(float4* hdr, const ObsDev* obs, const uint32_
         ay = ay + ry * DOWN_WB[j];
         az = az + rz * DOWN_WB[j];
     }
-    hdr[od.pyr_base + od.loff[k] + l] = make_float4(ax, ay, az, 0.0f);
+    return make_float4(ax, ay, az, 0.0f);
+}
+
+__global__ void k_bloom_down_batch(float4* hdr, const ObsDev* obs, const uint32_t* pre, uint32_t n, int k) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= __ldg(pre + n)) return;
+    uint32_t o = find_obs(pre, n, i);
+    const ObsDev& od = obs[o];
+    uint32_t l = i - __ldg(pre + o);
+    hdr[od.pyr_base + od.loff[k] + l] = bloom_down_px(hdr, od, k, l % od.lw[k], l / od.lw[k]);
 }
 
 __device__ __forceinline__ float4 upsample_b(const float4* c, uint32_t cw, uint32_t ch, uint32_t x, uint32_t y) {
@@ -63,6 +67,30 @@ __global__ void k_bloom_up_batch(float4* hdr, const ObsDev* obs, const uint32_t*
     float4* dst = hdr + od.pyr_base + od.loff[k] + l;
     float4 v = *dst;
     *dst = make_float4(v.x + up.x, v.y + up.y, v.z + up.z, 0.0f);
+}
+
+// The coarse levels of every observer, one block each: down to levels k0..6, then level k += up(level k + 1) for
+// 5..k0. A level of at most BLOOM_TAIL pixels keeps a block a few microseconds; as launches of their own the
+// eight passes from level 3 on took 4 us each whatever their size (12 launches and 53 us for a 320x200 frame).
+constexpr uint32_t BLOOM_TAIL = 20000;
+__global__ void __launch_bounds__(1024) k_bloom_tail_batch(float4* hdr, const ObsDev* obs, int k0) {
+    const ObsDev& od = obs[blockIdx.x];
+    for (int k = k0; k <= SR_BLOOM_LEVELS; ++k) {
+        const uint32_t w = od.lw[k], px = w * od.lh[k];
+        for (uint32_t l = threadIdx.x; l < px; l += blockDim.x)
+            hdr[od.pyr_base + od.loff[k] + l] = bloom_down_px(hdr, od, k, l % w, l / w);
+        __syncthreads();
+    }
+    for (int k = SR_BLOOM_LEVELS - 1; k >= k0; --k) {
+        const uint32_t w = od.lw[k], px = w * od.lh[k];
+        for (uint32_t l = threadIdx.x; l < px; l += blockDim.x) {
+            const float4 up = upsample_b(hdr + od.pyr_base + od.loff[k + 1], od.lw[k + 1], od.lh[k + 1], l % w, l / w);
+            float4* dst = hdr + od.pyr_base + od.loff[k] + l;
+            const float4 v = *dst;
+            *dst = make_float4(v.x + up.x, v.y + up.y, v.z + up.z, 0.0f);
+        }
+        __syncthreads();
+    }
 }
 
 // The composite (bloom.rs:93-125) and pack_rgb_with_lut (renderer.rs:1116-1129) of every pixel of

@@ -285,9 +285,13 @@ __device__ __forceinline__ Cam cam_of(const float4* cam, uint32_t o) {
     return r;
 }
 
+// The observers of a batch; also clears the batch's counters (no launch of their own).
 __global__ void k_camera_batch(uint32_t n, const SrGpuUniforms* U, const SrCameraF64* cam64, const ObsDev* obs,
-                               double a0, double a1, double a2, double a3, float4* cam) {
+                               double a0, double a1, double a2, double a3, float4* cam, uint32_t* counters,
+                               uint32_t num_counters, uint32_t* sched, uint32_t num_sched) {
     uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t k = o; k < num_counters; k += gridDim.x * blockDim.x) counters[k] = 0u;
+    for (uint32_t k = o; k < num_sched; k += gridDim.x * blockDim.x) sched[k] = 0u;
     if (o >= n) return;
     float4* out = cam + 6ull * o;
     if (obs[o].has_cam64) {
@@ -1575,6 +1579,10 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                               cudaStream_t st) {
     if (r.n == 0) return cudaSuccess;
     c.adj_valid = false;  // the batch buffers the gradient's outcomes live in are about to change
+    auto drop_graphs = [&]() {  // their last launches may still run
+        cudaStreamSynchronize(st);
+        fast_release(c);
+    };
     // The packet walk; counting runs take the per-lane order, whose work counts are the reference's.
     bool packet = t.packet != 0 && !r.count_work && (s.empty || s.fan_levels != 0);
     Shape sh;
@@ -1592,7 +1600,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         packet = sh.total_tiles < FAN_MAX_TILES &&
                  c.fan_list.ensure((size_t)sh.total_tiles * FAN_QUEUED_PER_TILE * 4) == cudaSuccess &&
                  c.fan_shadows.ensure((size_t)sh.total_tiles * FAN_SHADOWS_PER_TILE * 4) == cudaSuccess;
-        if (c.fan_list.bytes != old || c.fan_shadows.bytes != old_shadows) fast_release(c);
+        if (c.fan_list.bytes != old || c.fan_shadows.bytes != old_shadows) drop_graphs();
         if (c.fan_list.bytes != old && c.fan_list.p) {
             cudaError_t z = cudaMemsetAsync(c.fan_list.p, 0, c.fan_list.bytes, st);
             if (z != cudaSuccess) return z;
@@ -1608,12 +1616,13 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     if ((uint64_t)sh.total_tiles * 32 >= (1ull << 32)) return cudaErrorInvalidValue;
     cudaError_t e;
     // Buffers (grown on demand; a growth invalidates every captured graph).
-    size_t old_hits = c.hits.bytes, old_hdr = c.hdr.bytes, old_U = c.U.bytes, old_sh = c.shadow.bytes, old_rgb = c.rgb.bytes;
-    if ((e = c.U.ensure(n * sizeof(SrGpuUniforms))) != cudaSuccess) return e;
-    if ((e = c.cam64.ensure(n * sizeof(SrCameraF64))) != cudaSuccess) return e;
+    size_t old_hits = c.hits.bytes, old_hdr = c.hdr.bytes, old_U = c.inputs.bytes, old_sh = c.shadow.bytes, old_rgb = c.rgb.bytes;
+    // The batch's inputs are one block, copied at once: uniforms, cameras, observers, prefix rows.
+    const size_t at_cam = n * sizeof(SrGpuUniforms), at_obs = at_cam + n * sizeof(SrCameraF64);
+    const size_t at_pre = at_obs + n * sizeof(ObsDev), in_bytes = at_pre + sh.pre.size() * 4;
+    static_assert(sizeof(SrGpuUniforms) % 16 == 0 && sizeof(SrCameraF64) % 8 == 0 && sizeof(ObsDev) % 8 == 0, "the block's parts stay aligned");
+    if ((e = c.inputs.ensure(in_bytes)) != cudaSuccess) return e;
     if ((e = c.cam.ensure(n * 6 * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = c.obs.ensure(n * sizeof(ObsDev))) != cudaSuccess) return e;
-    if ((e = c.lvl_pre.ensure(sh.pre.size() * 4)) != cudaSuccess) return e;
     if ((e = c.hits.ensure((size_t)sh.total_px * sizeof(float4))) != cudaSuccess) return e;
     if ((e = c.slots.ensure((size_t)sh.total_px * 4)) != cudaSuccess) return e;
     if ((e = c.shadow.ensure((size_t)sh.total_px)) != cudaSuccess) return e;  // shadow states
@@ -1644,54 +1653,62 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         if ((e = c.star_r.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
         if ((e = c.star_color.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
         if ((e = c.star_box.ensure(pairs * sizeof(float4))) != cudaSuccess) return e;
-        if ((e = c.star_count.ensure(tiles * 4)) != cudaSuccess) return e;
+        if ((e = c.star_count.ensure(2 * tiles * 4)) != cudaSuccess) return e;
         if ((e = c.star_offset.ensure(tiles * 4)) != cudaSuccess) return e;
-        if ((e = c.star_fill.ensure(tiles * 4)) != cudaSuccess) return e;
         if ((e = c.star_list.ensure((size_t)list_cap * 4)) != cudaSuccess) return e;
         if ((e = c.star_scan.ensure(scan_bytes)) != cudaSuccess) return e;
     }
     if (c.star_r.bytes + c.star_box.bytes + c.star_count.bytes + c.star_list.bytes + c.star_scan.bytes != old_star)
-        fast_release(c);
+        drop_graphs();
     if (!r.rgb && (e = c.rgb.ensure((size_t)sh.total_px * 4)) != cudaSuccess) return e;
-    if ((e = c.hU.ensure(n * sizeof(SrGpuUniforms))) != cudaSuccess) return e;
-    if ((e = c.hcam64.ensure(n * sizeof(SrCameraF64))) != cudaSuccess) return e;
-    if ((e = c.hobs.ensure(n * sizeof(ObsDev))) != cudaSuccess) return e;
-    if ((e = c.hlvl.ensure(sh.pre.size() * 4)) != cudaSuccess) return e;
-    if (c.hits.bytes != old_hits || c.hdr.bytes != old_hdr || c.U.bytes != old_U || c.shadow.bytes != old_sh ||
+    if (c.hits.bytes != old_hits || c.hdr.bytes != old_hdr || c.inputs.bytes != old_U || c.shadow.bytes != old_sh ||
         c.rgb.bytes != old_rgb)
-        fast_release(c);
-    // The previous batch's copies from the pinned staging must have run before it is rewritten.
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-    std::memcpy(c.hU.p, r.u, n * sizeof(SrGpuUniforms));
-    if (r.cam64) std::memcpy(c.hcam64.p, r.cam64, n * sizeof(SrCameraF64));
-    std::memcpy(c.hobs.p, sh.obs.data(), n * sizeof(ObsDev));
-    std::memcpy(c.hlvl.p, sh.pre.data(), sh.pre.size() * 4);
+        drop_graphs();
+    // Two pinned staging blocks in turn, so that a call does not wait for the batch before it: a block is
+    // rewritten once the copy from it, two calls ago, has run.
+    const int slot = c.staging_next;
+    c.staging_next = 1 - slot;
+    if (!c.staged[slot] && (e = cudaEventCreateWithFlags(&c.staged[slot], cudaEventDisableTiming)) != cudaSuccess) return e;
+    if ((e = cudaEventSynchronize(c.staged[slot])) != cudaSuccess) return e;
+    if ((e = c.staging[slot].ensure(in_bytes)) != cudaSuccess) return e;
+    unsigned char* host = c.staging[slot].as<unsigned char>();
+    std::memcpy(host, r.u, n * sizeof(SrGpuUniforms));
+    if (r.cam64) std::memcpy(host + at_cam, r.cam64, n * sizeof(SrCameraF64));
+    std::memcpy(host + at_obs, sh.obs.data(), n * sizeof(ObsDev));
+    std::memcpy(host + at_pre, sh.pre.data(), sh.pre.size() * 4);
+    unsigned char* dev = c.inputs.as<unsigned char>();
+    if ((e = cudaMemcpyAsync(dev, host, in_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
+    if ((e = cudaEventRecord(c.staged[slot], st)) != cudaSuccess) return e;
+    struct {
+        const SrGpuUniforms* U;
+        const SrCameraF64* cam64;
+        const ObsDev* obs;
+        const uint32_t* pre;
+    } in{reinterpret_cast<const SrGpuUniforms*>(dev), reinterpret_cast<const SrCameraF64*>(dev + at_cam),
+         reinterpret_cast<const ObsDev*>(dev + at_obs), reinterpret_cast<const uint32_t*>(dev + at_pre)};
+    c.batch_U = in.U;
+    c.batch_obs = in.obs;
 
     uint32_t* rgb = r.rgb ? r.rgb : c.rgb.as<uint32_t>();
     const WideScene ws = wide_scene(s, sd);
     unsigned long long* work = reinterpret_cast<unsigned long long*>(counters + 4);
-    const uint32_t* tile_pre = c.lvl_pre.as<uint32_t>();
+    const uint32_t* tile_pre = in.pre;
     const uint32_t* pix_pre = tile_pre + stride;
 
     auto sequence = [&](bool timed) -> cudaError_t {
         cudaError_t x;
-        if ((x = cudaMemcpyAsync(c.U.p, c.hU.p, n * sizeof(SrGpuUniforms), cudaMemcpyHostToDevice, st)) != cudaSuccess) return x;
-        if (r.cam64 && (x = cudaMemcpyAsync(c.cam64.p, c.hcam64.p, n * sizeof(SrCameraF64), cudaMemcpyHostToDevice, st)) != cudaSuccess) return x;
-        if ((x = cudaMemcpyAsync(c.obs.p, c.hobs.p, n * sizeof(ObsDev), cudaMemcpyHostToDevice, st)) != cudaSuccess) return x;
-        if ((x = cudaMemcpyAsync(c.lvl_pre.p, c.hlvl.p, sh.pre.size() * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) return x;
-        if ((x = cudaMemsetAsync(counters, 0, r.count_work ? 64 : 16, st)) != cudaSuccess) return x;
-        if ((x = cudaMemsetAsync(c.sched.p, 0, c.sched.bytes, st)) != cudaSuccess) return x;
-        k_camera_batch<<<(n + 63) / 64, 64, 0, st>>>(n, c.U.as<SrGpuUniforms>(), c.cam64.as<SrCameraF64>(), c.obs.as<ObsDev>(),
-                                                     anchor[0], anchor[1], anchor[2], anchor[3], c.cam.as<float4>());
+        k_camera_batch<<<(n + 63) / 64, 64, 0, st>>>(n, in.U, in.cam64, in.obs, anchor[0], anchor[1], anchor[2], anchor[3],
+                                                     c.cam.as<float4>(), counters, r.count_work ? 16u : 4u,
+                                                     c.sched.as<uint32_t>(), (uint32_t)(c.sched.bytes / 4));
         if (timed) cudaEventRecord(r.ev[0], st);
         TraceBatchArgs ta;
         ta.top_n = 0;
         ta.ws = ws;
         ta.attrs = sd.attrs;
         ta.mats = sd.mats;
-        ta.U = c.U.as<SrGpuUniforms>();
+        ta.U = in.U;
         ta.cam = c.cam.as<float4>();
-        ta.obs = c.obs.as<ObsDev>();
+        ta.obs = in.obs;
         ta.tile_pre = tile_pre;
         ta.n = n;
         ta.total_rays = sh.total_tiles * 32u;
@@ -1781,8 +1798,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         if (timed) cudaEventRecord(r.ev[2], st);
         if (binned) {
             const size_t tiles = sh.total_star_tiles;
-            if ((x = cudaMemsetAsync(c.star_count.p, 0, tiles * 4, st)) != cudaSuccess) return x;
-            if ((x = cudaMemsetAsync(c.star_fill.p, 0, tiles * 4, st)) != cudaSuccess) return x;
+            if ((x = cudaMemsetAsync(c.star_count.p, 0, 2 * tiles * 4, st)) != cudaSuccess) return x;  // counts and cursors
             StarBinArgs ba;
             ba.U = sa.U;
             ba.cam = sa.cam;
@@ -1796,7 +1812,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
             ba.bb = bb;
             ba.count = c.star_count.as<uint32_t>();
             ba.offset = c.star_offset.as<uint32_t>();
-            ba.fill = c.star_fill.as<uint32_t>();
+            ba.fill = ba.count + tiles;
             ba.list = c.star_list.as<uint32_t>();
             ba.list_cap = list_cap;
             const uint64_t pairs = (uint64_t)n * sd.num_stars;
@@ -1831,12 +1847,16 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         }
         if (timed) cudaEventRecord(r.ev[3], st);
         if (r.no_image) return cudaSuccess;
-        for (int k = 1; k <= SR_BLOOM_LEVELS; ++k) {
+        int tail = 1;  // the first level that one block per observer takes
+        for (uint32_t i = 0; i < n; ++i)
+            while (tail <= SR_BLOOM_LEVELS && sh.obs[i].lw[tail] * sh.obs[i].lh[tail] > BLOOM_TAIL) ++tail;
+        for (int k = 1; k < tail; ++k) {
             const uint32_t* pre = tile_pre + (size_t)(1 + k) * stride;
             uint32_t tot = sh.pre[(size_t)(1 + k) * stride + n];
             k_bloom_down_batch<<<(tot + 255) / 256, 256, 0, st>>>(sa.hdr, sa.obs, pre, n, k);
         }
-        for (int k = SR_BLOOM_LEVELS - 1; k >= 1; --k) {
+        if (tail <= SR_BLOOM_LEVELS) k_bloom_tail_batch<<<n, 1024, 0, st>>>(sa.hdr, sa.obs, tail);
+        for (int k = std::min(tail, SR_BLOOM_LEVELS) - 1; k >= 1; --k) {
             const uint32_t* pre = tile_pre + (size_t)(1 + k) * stride;
             uint32_t tot = sh.pre[(size_t)(1 + k) * stride + n];
             k_bloom_up_batch<<<(tot + 255) / 256, 256, 0, st>>>(sa.hdr, sa.obs, pre, n, k);
@@ -1872,7 +1892,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     for (auto& o : sh.obs) key = mix(key, ((uint64_t)o.width << 32) | o.height);
     auto it = c.graphs.find(key);
     if (it == c.graphs.end()) {
-        if (c.graphs.size() > 64) fast_release(c);
+        if (c.graphs.size() > 64) drop_graphs();
         GraphEntry g;
         if ((e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return sequence(false);
         cudaError_t se = sequence(false);
@@ -1986,8 +2006,8 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
                                                                   c.adj_cam.as<DCam>(), bb, c.adj_stars.as<float>());
     AdjointArgs a;
     a.s = sd;
-    a.U = c.U.as<SrGpuUniforms>();
-    a.obs = c.obs.as<ObsDev>();
+    a.U = c.batch_U;
+    a.obs = c.batch_obs;
     a.star_pre = nullptr;
     a.dcam = c.adj_cam.as<DCam>();
     a.hits = c.hits.as<float4>();

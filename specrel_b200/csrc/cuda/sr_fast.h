@@ -102,10 +102,11 @@ struct FastCtx {
     // shadow: one byte per pixel, the main light's shadow ray as traced (0 none, 1 clear, 2 occluded)
     // sched: the tile counters of the trace kernel, one per SM band then the shared pool's
     // fan_list, fan_shadows: the packet walk's queue, and its list of pixels that cast shadow rays
-    DevMem U, cam64, cam, obs, lvl_pre, hits, slots, shadow, hdr, rgb, sched, fan_list, fan_shadows;
+    // inputs: the batch's uniforms, cameras, observers and prefix rows
+    DevMem inputs, cam, hits, slots, shadow, hdr, rgb, sched, fan_list, fan_shadows;
     // Star binning: per (observer, star) the event in the observer's space, the colour and the footprint's box;
     // per 16x16 tile a count, a list offset and a fill cursor; the lists; the prefix sum's scratch.
-    DevMem star_r, star_color, star_box, star_count, star_offset, star_fill, star_list, star_scan;
+    DevMem star_r, star_color, star_box, star_count, star_offset, star_list, star_scan;
     // Gradient: the camera and the stars' cone events as duals, per-block partial sums, the result.
     // adj_star_sum, adj_star_n: per pixel the star sum's duals and how many terms it has.
     DevMem adj_cam, adj_stars, adj_partials, adj_out, adj_pyr, adj_weight, adj_grid, adj_pass, adj_hdr, adj_star_sum, adj_star_n;
@@ -114,8 +115,12 @@ struct FastCtx {
     bool adj_valid = false;
     uint32_t adj_w = 0, adj_h = 0, adj_level = 0, adj_r0 = 0, adj_r1 = 0;  // the last gradient call's frame and band
     const float4* adj_geoms = nullptr;
-    HostMem hU, hcam64, hobs, hlvl;
-    uint32_t cap_obs = 0;
+    HostMem staging[2];                 // pinned, in turn
+    cudaEvent_t staged[2] = {nullptr, nullptr};  // the last copy from each has run
+    int staging_next = 0;
+    const SrGpuUniforms* batch_U = nullptr;  // the last batch's, on the device
+    const ObsDev* batch_obs = nullptr;
+    ~FastCtx() { for (cudaEvent_t e : staged) if (e) cudaEventDestroy(e); }
     std::map<uint64_t, GraphEntry> graphs;
 };
 
