@@ -847,7 +847,16 @@ struct FanTasks {
     uint32_t waste;     // FAN_WASTE or FAN_WASTE_SMALL
 };
 
-// log2 of a tile's pixels: 64, fewer where that leaves less than a tile or so per warp.
+// Launches whose rays walk alone (k_trace_lean) all the same: few of them through a small scene, where no
+// walk is long and the packet's two launches, bounds and queue cost more than they save. Trace time, lone
+// against packet: 37k tetrahedra, 320x200: 13 against 30 us, 16 frames of about that size 110 against 231, 8 of
+// 640x400 142 against 242, but 1920x1200 88 against 65; 111k, 320x200: 18 against 34, 8 of 640x400 194 against
+// 305; 147k, 640x400: 69 against 61, four of them 267 against 211.
+static bool lone_rays(uint64_t prims, uint64_t pixels) { return prims <= 1u << 17 && prims * pixels < 1ull << 36; }
+
+// log2 of a tile's pixels: 64, fewer where that leaves less than a tile or so per warp (one 120x78 frame of
+// three: 0.23 ms in tiles of 64, 0.11 in tiles of 8; the 1280x800 frame of the 7.9M-tet workload: 0.29 ms in
+// tiles of 64).
 static uint32_t fan_tile_log(uint64_t pixels) { return pixels < (128u << 10) ? 3u : (pixels < (512u << 10) ? 4u : 6u); }
 
 __device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
@@ -1068,15 +1077,15 @@ __global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchAr
     FanQueue& sm = sm_queue[threadIdx.x >> 5];
     uint2 st[FAN_LEVELS];
     const uint32_t tiles = a.total_rays >> 5, tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t mine = 0, ahead = 0;  // ahead: the next tile, asked for a tile early (lane 0)
-    if (lane == 0) ahead = atomicAdd(q.count + FAN_NEXT, 1u);
+    const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
+    // ahead: the next tile, the warp's own number first, then asked for a tile early (lane 0).
+    uint32_t mine = 0, ahead = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     bool whole = true;  // whole tiles first, then the queue
     for (;;) {
         uint32_t tile, part = 0;
         if (whole) {
             tile = __shfl_sync(FULL_WARP, ahead, 0);
-            if (lane == 0 && tile < tiles) ahead = atomicAdd(q.count + FAN_NEXT, 1u);
+            if (lane == 0 && tile < tiles) ahead = warps + atomicAdd(q.count + FAN_NEXT, 1u);
             if (tile >= tiles) {
                 fan_first_done(q, mine);
                 whole = false;
@@ -1125,6 +1134,7 @@ __global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ Trac
     uint2 st[FAN_LEVELS];
     const uint32_t tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
     const uint32_t tasks = *q.num_shadows, part_mask = (1u << FAN_PARTS_LOG) - 1u;
+    if (tasks == 0) return;
     uint32_t mine = 0;
     for (;;) {
         const uint32_t next = warp_next(q.count + FAN_NEXT);
@@ -1584,13 +1594,13 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         fast_release(c);
     };
     // The packet walk; counting runs take the per-lane order, whose work counts are the reference's.
-    bool packet = t.packet != 0 && !r.count_work && (s.empty || s.fan_levels != 0);
+    uint64_t pixels = 0;
+    for (uint32_t i = 0; i < r.n; ++i) pixels += (uint64_t)r.u[i].size[0] * r.u[i].size[1];
+    bool packet = t.packet != 0 && !r.count_work && (s.empty || s.fan_levels != 0) && !lone_rays(sd.num_prims, pixels);
     Shape sh;
     uint32_t tile_w = t.tile_w, tile_h = t.tile_h;
     if (packet) {
-        uint64_t pixels = 0;
-        for (uint32_t i = 0; i < r.n; ++i) pixels += (uint64_t)r.u[i].size[0] * r.u[i].size[1];
-        const uint32_t size_log = getenv("FAN_T") ? atoi(getenv("FAN_T")) : fan_tile_log(pixels);
+        const uint32_t size_log = fan_tile_log(pixels);
         (tile_w < tile_h ? tile_w : tile_h) *= 2;
         while (tile_w * tile_h > (1u << size_log)) (tile_w > tile_h ? tile_w : tile_h) /= 2;
         sh = make_shape(r, tile_w, tile_h);

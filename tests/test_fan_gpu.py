@@ -79,7 +79,8 @@ def test_shadow_rays(engine, bodies, shadow):
 def test_large_leaves(engine, bodies, group):
     """The same records under trees over groups of `group` of them, so that leaves hold up to 63: more than a
     warp has lanes, and all a node reference can name."""
-    boxes, geoms, attrs, p = sr.synth_scene(1, 5, n_bodies=8, steps=16).build_inputs()
+    boxes, geoms, attrs, p = sr.synth_scene(1, 5, n_bodies=64).build_inputs()  # too large for small frames' own walk
+    assert len(geoms) > 1 << 17
     n = len(geoms)
     starts = np.arange(0, n, group)
     lo = np.minimum.reduceat(boxes[:, :4], starts, axis=0)
@@ -108,6 +109,18 @@ def test_large_leaves(engine, bodies, group):
         u = sr.uniforms(cam, 203, 117, 0, 1, 0, num_nodes=len(nodes), light_pos=p.light_pos)
         seen += int((_both(engine, BIG, u, None).hit_id != 0xFFFFFFFF).sum())
     assert seen > 0
+
+
+@pytest.mark.parametrize("side", [-2, 2])
+def test_small_scene_either_side_of_the_line(engine, side):
+    """36,864 records: their rays walk alone up to 2^36 / 36,864 pixels a launch, as packets from there on."""
+    s = sr.synth_scene(1, 1, n_bodies=16)
+    engine.build_tubes(BIG, s)
+    edge = 2**36 / engine.stats(BIG).num_prims
+    w, h = 1366, int(edge / 1366) + side
+    assert (w * h < edge) == (side < 0)
+    u, cam = _u(s, w, h, (0.3, -0.2, 0.4))
+    assert (_both(engine, BIG, u, cam).hit_id != 0xFFFFFFFF).any()
 
 
 def test_frames_of_growing_size_in_turn(engine, bodies):
