@@ -1077,15 +1077,17 @@ __global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchAr
     FanQueue& sm = sm_queue[threadIdx.x >> 5];
     uint2 st[FAN_LEVELS];
     const uint32_t tiles = a.total_rays >> 5, tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
-    const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
-    // ahead: the next tile, the warp's own number first, then asked for a tile early (lane 0).
-    uint32_t mine = 0, ahead = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    // ahead: the next tile, asked for a tile early (lane 0). No tile belongs to a warp by its number: those
+    // that wait must wait for running warps only, and a block may start late where other launches run.
+    uint32_t mine = 0, ahead = 0;
+    if (lane == 0) ahead = atomicAdd(q.count + FAN_NEXT, 1u);
     bool whole = true;  // whole tiles first, then the queue
     for (;;) {
         uint32_t tile, part = 0;
         if (whole) {
             tile = __shfl_sync(FULL_WARP, ahead, 0);
-            if (lane == 0 && tile < tiles) ahead = warps + atomicAdd(q.count + FAN_NEXT, 1u);
+            if (lane == 0 && tile < tiles) ahead = atomicAdd(q.count + FAN_NEXT, 1u);
             if (tile >= tiles) {
                 fan_first_done(q, mine);
                 whole = false;
