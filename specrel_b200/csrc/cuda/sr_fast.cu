@@ -817,8 +817,10 @@ __global__ void __launch_bounds__(512) k_trace_lean(const __grid_constant__ Trac
 // cycles per instruction against 0.2 of 7).
 //
 // The queue: an entry is written at list[tail++]; a warp takes the ticket head++, and the entry of that
-// number is its next task, or there is none once all first tasks and every entry are finished. A warp
-// waits only for work that others are doing, which never waits for it, and for at most FAN_POLLS polls.
+// number is its next task, or there is none once all first tasks and every entry are finished. Only the warps
+// of the first blocks (`helpers`) do so while the queue is empty; the others leave then (a warp that queued
+// something comes back for it itself). A warp waits only for work that running warps are doing, which never
+// waits for it, and for at most FAN_POLLS polls.
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t FAN_BUDGET = 400, FAN_ANY_BUDGET = 160;
 // Tests without a hit after which a tile's walk is given up. A walk given up costs more in parts (from
@@ -830,6 +832,12 @@ constexpr uint32_t FAN_WASTE = 256, FAN_WASTE_SMALL = 128, FAN_SMALL_TILES = 48u
 constexpr uint32_t FAN_UNLIMITED = 1u << 22;
 constexpr uint32_t FAN_GROUP_LOG = 3, FAN_PAIR_LOG = 1;  // log2 of a group's and a pair's pixels
 constexpr uint32_t FAN_POLLS = 1u << 21;
+// Blocks that stay for the queue: one for every 4 SMs. Waiting warps hold the room that another stream's launch
+// could use and their polls slow the working ones. With three engines' frames in turn, all blocks waiting against a
+// quarter of the SMs' number against none: 1280x800 of the 7.9M-tet workload 738, 410 and 452 us a frame, five
+// frames of 471x163 to 715x513 656, 338 and 358, 8 of 1280x800 3.02, 2.79 and 2.78 ms; one engine alone, trace
+// time: 294, 259 and 251 us (1280x800, 16 bodies), 580, 608 and 623 (the five).
+constexpr uint32_t FAN_HELPERS_PER = 4;
 // A task: tile * 64 + part + 1 (0: no entry yet). Parts of a tile in k_fan_trace's queue: its 8 groups of 8
 // pixels, then its 32 pairs; in the list of shadow rays: its two halves of 32 pixels, then its 8 groups, then
 // its 32 pairs; in k_fan_shadow's queue: its 64 pixels.
@@ -845,6 +853,7 @@ struct FanTasks {
     uint32_t* shadows;  // the pixels that cast shadow rays, as tasks
     uint32_t* num_shadows;
     uint32_t waste;     // FAN_WASTE or FAN_WASTE_SMALL
+    uint32_t helpers;   // the first blocks, whose warps wait for the queue's entries
 };
 
 // Launches whose rays walk alone (k_trace_lean) all the same: few of them through a small scene, where no
@@ -912,7 +921,8 @@ __device__ __forceinline__ void fan_finished(const FanTasks& q) {
 // The next task of the queue, or 0 when all work is done (`first`: the number of first tasks).
 __device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, uint32_t* err) {
     uint32_t entry = 0;
-    if ((threadIdx.x & 31u) == 0) {
+    if ((threadIdx.x & 31u) == 0 &&
+        (blockIdx.x < q.helpers || (int)(load_acquire(q.count + FAN_TAIL) - load_acquire(q.count + FAN_HEAD)) > 0)) {
         const uint32_t ticket = atomicAdd(q.count + FAN_HEAD, 1u);
         for (uint32_t polls = 0;; ++polls) {
             if (load_acquire(q.count + FAN_TAIL) > ticket) {
@@ -1758,6 +1768,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                 ft.num_shadows = ft.count + 2 * FAN_COUNTERS;
                 ft.list = c.fan_list.as<uint32_t>();
                 ft.shadows = c.fan_shadows.as<uint32_t>();
+                ft.helpers = (uint32_t)c.num_sms / FAN_HELPERS_PER;
                 ft.waste = sh.total_tiles < FAN_SMALL_TILES ? FAN_WASTE_SMALL : FAN_WASTE;
                 const uint32_t warps = t.block_threads / 32;
                 if (oct) k_fan_trace<true><<<blocks, t.block_threads, warps * sizeof(FanQueue), st>>>(ta, ft);
