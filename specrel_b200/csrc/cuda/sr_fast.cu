@@ -863,10 +863,10 @@ struct FanTasks {
 // 305; 147k, 640x400: 69 against 61, four of them 267 against 211.
 static bool lone_rays(uint64_t prims, uint64_t pixels) { return prims <= 1u << 17 && prims * pixels < 1ull << 36; }
 
-// log2 of a tile's pixels: 64, fewer where that leaves less than a tile or so per warp (one 120x78 frame of
-// three: 0.23 ms in tiles of 64, 0.11 in tiles of 8; the 1280x800 frame of the 7.9M-tet workload: 0.29 ms in
-// tiles of 64).
-static uint32_t fan_tile_log(uint64_t pixels) { return pixels < (128u << 10) ? 3u : (pixels < (512u << 10) ? 4u : 6u); }
+// log2 of a tile's pixels: 64, or 8 where that leaves less than a tile per warp. Three engines' frames in turn, in
+// tiles of 8, 16 and 64: 16 accelerated bodies at 120x78 102, 138 and 151 us a frame, at 320x200 130, 152 and
+// 154, at 640x400 205, 181 and 163, at 1100x700 459, 285 and 185; 147k tetrahedra at 451x205 76, 82 and 93.
+static uint32_t fan_tile_log(uint64_t pixels) { return pixels < (128u << 10) ? 3u : 6u; }
 
 __device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
     uint32_t v;
