@@ -534,7 +534,8 @@ typedef struct SrTuning {
                                  long as every hit lies beyond its leaf box's computed entry
                                  parameter (the records' 1e-4 box padding keeps a margin of
                                  1e-4 / |d| in ray parameter against its rounding); with
-                                 stack_smem 0, top_levels 0 and the single-tile schedule.
+                                 stack_smem 0, top_levels 0 and the single-tile schedule. Launches
+                                 too small to gain by it take the per-ray order all the same.
                                  0: each ray walks the tree in its own near-first order (work
                                  counts, SR_FLAG_COUNT_WORK, always come from this order) */
 } SrTuning;

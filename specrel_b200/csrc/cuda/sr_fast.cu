@@ -4,7 +4,7 @@
 //   k_camera_batch   FP64 observers (tetrad from rapidity in double, event rebased to the anchor)
 //   k_fan_trace, k_fan_shadow   persistent traversal (the default): each warp walks the 64 rays of an
 //                    8x8-pixel tile as one packet (closest hits), then the main light's shadow rays.
-//   k_trace_lean     the same work ray by ray (SrTuning.packet = 0): warps take 32-ray tiles from a
+//   k_trace_lean     the same work ray by ray (SrTuning.packet = 0, and small launches): warps take 32-ray tiles from a
 //                    global counter; each lane traces its pixel's primary ray, then its shadow ray.
 //   k_trace_batch    the same work under the other schedules of SrTuning (per-warp chunks of
 //                    tiles, partial refills, postponed or cooperative leaf tests).
@@ -233,7 +233,7 @@ SrTuning fast_default_tuning(const FastCtx& c) {
     (void)c;
     SrTuning t{};
     t.block_threads = 128;
-    t.blocks_per_sm = 8;  // the packet kernel's 64 registers leave room for 8 blocks of 128
+    t.blocks_per_sm = 8;  // the packet kernels take as many of these as are resident (fan_blocks)
     t.tile_w = 4;
     t.tile_h = 8;
     t.chunk_tiles = 1;
@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(512) k_trace_lean(const __grid_constant__ Trac
 // ---------------------------------------------------------------------------------------------
 // The packet form (SrTuning.packet): the walks of sr_fan.cuh in two persistent launches.
 //
-//   k_fan_trace    Every warp takes 8x8-pixel tiles (64 rays, two per lane) until there are none. A walk
+//   k_fan_trace    Every warp takes tiles of 64 pixels (two rays per lane; 8 pixels in small frames) until there are none. A walk
 //                  of more than FAN_BUDGET steps is given up: its tile goes into a queue as eight
 //                  groups of 8 pixels, which the warps walk from the hits found, as they run out of tiles.
 //                  Pixels whose hits cast a shadow ray are listed, 32 (or a group) at a time.

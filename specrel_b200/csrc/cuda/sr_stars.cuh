@@ -186,7 +186,7 @@ struct StarTileArgs {
 // passed round by shuffles, so that the terms, which must be added one after the other, wait for no
 // memory. It is bound by the densest tiles' chains: a block takes a quarter of a tile, so that they
 // spread over the chip. 100k stars at 1280x800: 162 us for 16x16 pixels a block with the sort and a
-// star's whole term per pixel.
+// star's whole term per pixel; 51 us, and 20 for the sort, like this.
 constexpr uint32_t STAR_BLOCKS = 4;  // blocks of two warps per tile
 __global__ void __launch_bounds__(64) k_star_tiles(const __grid_constant__ StarTileArgs a) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
