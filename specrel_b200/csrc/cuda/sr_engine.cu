@@ -155,8 +155,18 @@ sr_status sr_set_stream(sr_ctx* ctx, void* s) {
 }  // extern "C"
 
 namespace {
+// A wait in the packet walk's queue that ran out, in the frame of these flags or in an earlier one whose flags no
+// call has read (frames that stay on the device): reported once.
+sr_status queue_errors(sr_ctx* ctx, uint32_t flags) {
+    volatile uint32_t* lost = ctx->fast.fan_lost.as<uint32_t>();
+    if (!(flags & ERR_QUEUE_WAIT) && !*lost) return SR_OK;
+    *lost = 0;
+    return fail(ctx, SR_ERR_CUDA, "internal error: a wait in the trace kernel's queue ran out, a frame is incomplete");
+}
+
 // The device error flags a batch left in its counters (counters[1]), as a status.
 sr_status batch_errors(sr_ctx* ctx, uint32_t flags) {
+    if (sr_status r = queue_errors(ctx, flags); r != SR_OK) return r;
     if (flags & ERR_TRAVERSAL_LIMIT) return fail(ctx, SR_ERR_TRAVERSAL_LIMIT, "a ray exceeded the traversal visit limit");
     if (flags & ERR_SHADOW_MISMATCH) return fail(ctx, SR_ERR_CUDA, "internal error: shadow state mismatch");
     if (flags) return fail(ctx, SR_ERR_BAD_SCENE, "device reported a bad index");
@@ -183,6 +193,7 @@ sr_status sr_synchronize(sr_ctx* ctx) {
         const sr_status r = settle_async(ctx, (ctx->async.next + k) & 1);
         if (first == SR_OK) first = r;
     }
+    if (first == SR_OK) first = queue_errors(ctx, 0);
     return first;
 }
 
@@ -630,9 +641,24 @@ sr_status sr_render_ex(sr_ctx* ctx, uint32_t idx, const SrGpuUniforms* u, const 
             cudaEventElapsedTime(&timings->bloom_ms, ev[4], ev[5]);
         }
     }
+    if (sr_status r = queue_errors(ctx, counters[1]); r != SR_OK) return r;
     if (counters[1] & ERR_TRAVERSAL_LIMIT) return fail(ctx, SR_ERR_TRAVERSAL_LIMIT, "a ray exceeded the traversal visit limit");
     if (counters[1] & ERR_SHADOW_MISMATCH) return fail(ctx, SR_ERR_CUDA, "internal error: shadow state mismatch");
     if (counters[1]) return fail(ctx, SR_ERR_BAD_SCENE, "device reported a bad index (flags " + std::to_string(counters[1]) + ")");
+    return SR_OK;
+}
+
+sr_status sr_test_queue_polls(sr_ctx* ctx, uint32_t polls) {
+    if (!ctx) return SR_ERR_INVALID_ARGUMENT;
+    CK(cudaStreamSynchronize(ctx->stream), "synchronize");
+    fast_release(ctx->fast);  // the graphs hold the limit
+    ctx->fast.fan_polls = polls;
+    return SR_OK;
+}
+
+sr_status sr_test_queued(sr_ctx* ctx, uint32_t queued[2]) {
+    if (!ctx || !queued) return SR_ERR_INVALID_ARGUMENT;
+    CK(fast_queued(ctx->fast, queued, ctx->stream), "queue counts");
     return SR_OK;
 }
 
@@ -917,6 +943,7 @@ sr_status sr_adjoint_rows(sr_ctx* ctx, uint32_t idx, const SrGpuUniforms* u, con
        "gradient");
     uint32_t counters[4] = {0, 0, 0, 0};
     CK(cudaMemcpy(counters, ctx->counters.p, 16, cudaMemcpyDeviceToHost), "counters");
+    if (sr_status r = queue_errors(ctx, counters[1]); r != SR_OK) return r;
     if (counters[1] & ERR_TRAVERSAL_LIMIT) return fail(ctx, SR_ERR_TRAVERSAL_LIMIT, "a ray exceeded the traversal visit limit");
     if (counters[1]) return fail(ctx, SR_ERR_BAD_SCENE, "device reported a bad index (flags " + std::to_string(counters[1]) + ")");
     out->loss = r[0];

@@ -107,3 +107,10 @@ sr_status upload_scene_rest(sr_ctx* ctx, SceneSlot& s, const SrBuildDesc* d);
 sr_status check_build_desc(sr_ctx* ctx, const SrBuildDesc* d, const SrGpuAttr* host_attrs, uint32_t n);
 
 }  // namespace sre
+
+// For this library's tests only (not part of the interface): the limit of a wait in the packet walk's queue
+// (FastCtx::fan_polls), and how many parts the two launches of the context's last frame queued.
+extern "C" {
+sr_status sr_test_queue_polls(sr_ctx* ctx, uint32_t polls);
+sr_status sr_test_queued(sr_ctx* ctx, uint32_t queued[2]);
+}

@@ -124,6 +124,11 @@ __global__ void k_wide_fill(const SrGpuNode* nodes, uint32_t n, const uint32_t* 
     refs[wi] = make_uint2(ref[0], ref[1]);
 }
 
+// The packet walk's counters, a line each for those that many warps change.
+// FAN_LIST_HEAD: words of fan_list before its entries, the first of them `dirty`.
+constexpr uint32_t FAN_LIST_HEAD = 32;
+enum { FAN_NEXT = 0, FAN_HEAD = 32, FAN_TAIL = 64, FAN_FINISHED = 96, FAN_FIRST_DONE = 97, FAN_COUNTERS = 128 };
+
 static cudaError_t lean_kernel_attrs(int max_smem);
 static cudaError_t fan_resident(int threads, int* blocks);
 bool lean_stack_supported(uint32_t s);
@@ -143,7 +148,20 @@ cudaError_t fast_init(FastCtx& c, const cudaDeviceProp& prop) {
         if (e != cudaSuccess) return e;
         c.fan_blocks[threads / 128] = (uint32_t)std::max(n, 1);
     }
+    cudaError_t e = c.fan_lost.ensure(64);
+    if (e != cudaSuccess) return e;
+    std::memset(c.fan_lost.p, 0, c.fan_lost.bytes);
     return lean_kernel_attrs(c.max_smem);
+}
+
+cudaError_t fast_queued(const FastCtx& c, uint32_t queued[2], cudaStream_t st) {
+    queued[0] = queued[1] = 0;
+    if (!c.sched.p) return cudaSuccess;
+    for (int k = 0; k < 2; ++k) {
+        cudaError_t e = cudaMemcpyAsync(queued + k, c.sched.as<uint32_t>() + (uint32_t)k * FAN_COUNTERS + FAN_TAIL, 4, cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaStreamSynchronize(st);
 }
 
 void fast_release(FastCtx& c) {
@@ -285,11 +303,18 @@ __device__ __forceinline__ Cam cam_of(const float4* cam, uint32_t o) {
     return r;
 }
 
-// The observers of a batch; also clears the batch's counters (no launch of their own).
+// The observers of a batch; also clears the batch's counters (no launch of their own), and the packet walk's
+// queue where a wait that ran out in an earlier batch left entries in it (fan_dirty, null: no queue yet).
 __global__ void k_camera_batch(uint32_t n, const SrGpuUniforms* U, const SrCameraF64* cam64, const ObsDev* obs,
                                double a0, double a1, double a2, double a3, float4* cam, uint32_t* counters,
-                               uint32_t num_counters, uint32_t* sched, uint32_t num_sched) {
+                               uint32_t num_counters, uint32_t* sched, uint32_t num_sched, uint32_t* fan_dirty,
+                               uint32_t* fan_list, size_t num_fan_list) {
     uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0 && fan_dirty && *fan_dirty) {
+        for (size_t k = threadIdx.x; k < num_fan_list; k += blockDim.x) fan_list[k] = 0u;
+        __syncthreads();
+        if (threadIdx.x == 0) *fan_dirty = 0u;
+    }
     for (uint32_t k = o; k < num_counters; k += gridDim.x * blockDim.x) counters[k] = 0u;
     for (uint32_t k = o; k < num_sched; k += gridDim.x * blockDim.x) sched[k] = 0u;
     if (o >= n) return;
@@ -820,7 +845,10 @@ __global__ void __launch_bounds__(512) k_trace_lean(const __grid_constant__ Trac
 // number is its next task, or there is none once all first tasks and every entry are finished. Only the warps
 // of the first blocks (`helpers`) do so while the queue is empty; the others leave then (a warp that queued
 // something comes back for it itself). A warp waits only for work that running warps are doing, which never
-// waits for it, and for at most FAN_POLLS polls.
+// waits for it, and for at most q.polls polls. Where a wait runs out all the same, its ticket is given up and the
+// entry written later at its place is taken by nobody: the frame is incomplete (ERR_QUEUE_WAIT, and `lost`, which
+// outlives the frame's own flags until a call reports it) and the list is not zero at the end. `dirty` says so to
+// the launches behind: the shadow launch leaves, the next batch's camera launch clears the list.
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t FAN_BUDGET = 400, FAN_ANY_BUDGET = 160;
 // Tests without a hit after which a tile's walk is given up. A walk given up costs more in parts (from
@@ -831,7 +859,6 @@ constexpr uint32_t FAN_BUDGET = 400, FAN_ANY_BUDGET = 160;
 constexpr uint32_t FAN_WASTE = 256, FAN_WASTE_SMALL = 128, FAN_SMALL_TILES = 48u << 10;
 constexpr uint32_t FAN_UNLIMITED = 1u << 22;
 constexpr uint32_t FAN_GROUP_LOG = 3, FAN_PAIR_LOG = 1;  // log2 of a group's and a pair's pixels
-constexpr uint32_t FAN_POLLS = 1u << 21;
 // Blocks that stay for the queue: one for every 4 SMs. Waiting warps hold the room that another stream's launch
 // could use and their polls slow the working ones. With three engines' frames in turn, all blocks waiting against a
 // quarter of the SMs' number against none: 1280x800 of the 7.9M-tet workload 738, 410 and 452 us a frame, five
@@ -844,12 +871,13 @@ constexpr uint32_t FAN_HELPERS_PER = 4;
 constexpr uint32_t FAN_PARTS_LOG = 6, FAN_GROUPS = 8, FAN_HALVES = 2;
 constexpr uint32_t FAN_MAX_TILES = 1u << (31u - FAN_PARTS_LOG);
 constexpr uint32_t FAN_SHADOWS_PER_TILE = 32, FAN_QUEUED_PER_TILE = 64;
-// Counters, a line each for those that many warps change.
-enum { FAN_NEXT = 0, FAN_HEAD = 32, FAN_TAIL = 64, FAN_FINISHED = 96, FAN_FIRST_DONE = 97, FAN_COUNTERS = 128 };
 
 struct FanTasks {
     uint32_t* count;    // FAN_COUNTERS words of this launch, zero at the start
     uint32_t* list;     // the queue, zero at the start and again at the end
+    uint32_t* dirty;    // entries were left in the list
+    uint32_t* lost;     // a frame is incomplete (pinned host memory)
+    uint32_t polls;     // a wait's limit
     uint32_t* shadows;  // the pixels that cast shadow rays, as tasks
     uint32_t* num_shadows;
     uint32_t waste;     // FAN_WASTE or FAN_WASTE_SMALL
@@ -918,8 +946,9 @@ __device__ __forceinline__ void fan_finished(const FanTasks& q) {
         atomicAdd(q.count + FAN_FINISHED, 1u);
     }
 }
-// The next task of the queue, or 0 when all work is done (`first`: the number of first tasks).
-__device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, uint32_t* err) {
+// The next task of the queue, or 0 when all work is done (`first`: the number of first tasks), of a launch of
+// `tiles` tiles.
+__device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, uint32_t tiles, uint32_t* err) {
     uint32_t entry = 0;
     if ((threadIdx.x & 31u) == 0 &&
         (blockIdx.x < q.helpers || (int)(load_acquire(q.count + FAN_TAIL) - load_acquire(q.count + FAN_HEAD)) > 0)) {
@@ -941,10 +970,16 @@ __device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, 
                 }
                 __nanosleep(200);
             }
-            if (polls > FAN_POLLS) {
-                atomicOr(err, ERR_BAD_INDEX);
+            if (polls > q.polls) {
+                atomicOr(err, ERR_QUEUE_WAIT);
+                *(volatile uint32_t*)q.dirty = 1u;
+                *(volatile uint32_t*)q.lost = 1u;
                 break;
             }
+        }
+        if (entry && (entry - 1u) >> FAN_PARTS_LOG >= tiles) {  // not this launch's: never followed
+            atomicOr(err, ERR_BAD_INDEX);
+            entry = 0;
         }
     }
     return __shfl_sync(FULL_WARP, entry, 0);
@@ -1104,7 +1139,7 @@ __global__ void __maxnreg__(96) k_fan_trace(const __grid_constant__ TraceBatchAr
             }
         }
         if (!whole) {
-            const uint32_t task = fan_take(q, tiles, a.err);
+            const uint32_t task = fan_take(q, tiles, tiles, a.err);
             if (!task) break;
             tile = (task - 1u) >> FAN_PARTS_LOG;
             part = (task - 1u) & ((1u << FAN_PARTS_LOG) - 1u);
@@ -1146,7 +1181,7 @@ __global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ Trac
     uint2 st[FAN_LEVELS];
     const uint32_t tw_log = (uint32_t)__ffs((int)a.tile_w) - 1u, th_log = (uint32_t)__ffs((int)a.tile_h) - 1u;
     const uint32_t tasks = *q.num_shadows, part_mask = (1u << FAN_PARTS_LOG) - 1u;
-    if (tasks == 0) return;
+    if (tasks == 0 || *q.dirty) return;
     uint32_t mine = 0;
     for (;;) {
         const uint32_t next = warp_next(q.count + FAN_NEXT);
@@ -1180,14 +1215,14 @@ __global__ void __launch_bounds__(512) k_fan_shadow(const __grid_constant__ Trac
     }
     fan_first_done(q, mine);
     for (;;) {
-        const uint32_t task = fan_take(q, tasks, a.err);
+        const uint32_t task = fan_take(q, tasks, a.total_rays >> 5, a.err);
         if (!task) break;
         const uint32_t i = (task - 1u) & part_mask;
         const FanTile t = fan_tile(a, (task - 1u) >> FAN_PARTS_LOG);
         const ObsDev& od = a.obs[t.obs];
         const uint32_t px = t.x + (i & ((1u << tw_log) - 1u)), py = t.y + (i >> tw_log), pix = od.pix_base + py * od.width + px;
         ShadowQuery s;
-        if (fan_query(a, t.obs, px, py, pix, &s)) {  // the same for every lane
+        if (px < od.width && py < od.height && fan_query(a, t.obs, px, py, pix, &s)) {  // the same for every lane
             const bool hit = any_fan_one(a.ws, s.no, s.d, s.t_min, s.t_max, st, a.err);
             if (lane == 0) a.shadow[pix] = hit ? 2 : 1;
         }
@@ -1620,7 +1655,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         // Without room for the queue the rays walk alone. The queue's own buffer: its entries are zero
         // between launches, whatever the next one's size, the list's are not.
         packet = sh.total_tiles < FAN_MAX_TILES &&
-                 c.fan_list.ensure((size_t)sh.total_tiles * FAN_QUEUED_PER_TILE * 4) == cudaSuccess &&
+                 c.fan_list.ensure((FAN_LIST_HEAD + (size_t)sh.total_tiles * FAN_QUEUED_PER_TILE) * 4) == cudaSuccess &&
                  c.fan_shadows.ensure((size_t)sh.total_tiles * FAN_SHADOWS_PER_TILE * 4) == cudaSuccess;
         if (c.fan_list.bytes != old || c.fan_shadows.bytes != old_shadows) drop_graphs();
         if (c.fan_list.bytes != old && c.fan_list.p) {
@@ -1721,7 +1756,9 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         cudaError_t x;
         k_camera_batch<<<(n + 63) / 64, 64, 0, st>>>(n, in.U, in.cam64, in.obs, anchor[0], anchor[1], anchor[2], anchor[3],
                                                      c.cam.as<float4>(), counters, r.count_work ? 16u : 4u,
-                                                     c.sched.as<uint32_t>(), (uint32_t)(c.sched.bytes / 4));
+                                                     c.sched.as<uint32_t>(), (uint32_t)(c.sched.bytes / 4),
+                                                     c.fan_list.as<uint32_t>(), c.fan_list.as<uint32_t>() + FAN_LIST_HEAD,
+                                                     c.fan_list.p ? c.fan_list.bytes / 4 - FAN_LIST_HEAD : 0);
         if (timed) cudaEventRecord(r.ev[0], st);
         TraceBatchArgs ta;
         ta.top_n = 0;
@@ -1766,7 +1803,10 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                 FanTasks ft;
                 ft.count = c.sched.as<uint32_t>();
                 ft.num_shadows = ft.count + 2 * FAN_COUNTERS;
-                ft.list = c.fan_list.as<uint32_t>();
+                ft.dirty = c.fan_list.as<uint32_t>();
+                ft.list = ft.dirty + FAN_LIST_HEAD;
+                ft.lost = c.fan_lost.as<uint32_t>();
+                ft.polls = c.fan_polls;
                 ft.shadows = c.fan_shadows.as<uint32_t>();
                 ft.helpers = (uint32_t)c.num_sms / FAN_HELPERS_PER;
                 ft.waste = sh.total_tiles < FAN_SMALL_TILES ? FAN_WASTE_SMALL : FAN_WASTE;

@@ -102,6 +102,10 @@ struct FastCtx {
     // shadow: one byte per pixel, the main light's shadow ray as traced (0 none, 1 clear, 2 occluded)
     // sched: the tile counters of the trace kernel, one per SM band then the shared pool's
     // fan_list, fan_shadows: the packet walk's queue, and its list of pixels that cast shadow rays
+    // fan_lost: pinned; not 0 once a wait of the walk's queue ran out, until a call has reported it. fan_polls: such
+    // a wait's limit (about a second).
+    HostMem fan_lost;
+    uint32_t fan_polls = 1u << 21;
     // inputs: the batch's uniforms, cameras, observers and prefix rows
     DevMem inputs, cam, hits, slots, shadow, hdr, rgb, sched, fan_list, fan_shadows;
     // Star binning: per (observer, star) the event in the observer's space, the colour and the footprint's box;
@@ -126,6 +130,8 @@ struct FastCtx {
 
 cudaError_t fast_init(FastCtx& c, const cudaDeviceProp& prop);
 void fast_release(FastCtx& c);
+// How many parts the last packet frame's two launches queued.
+cudaError_t fast_queued(const FastCtx& c, uint32_t queued[2], cudaStream_t st);
 // Builds the layout from the device copy of the reference nodes. The scene is usable on the fast
 // path when its depth is <= 60 (the reference's stack never overflows), it has fewer than 2^25
 // primitives and every leaf holds at most 63 (the packed references); otherwise `usable` is false.

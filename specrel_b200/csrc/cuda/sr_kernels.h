@@ -47,6 +47,8 @@ constexpr uint32_t ERR_BAD_INDEX = 4u;
 // The fast path's shading asked for a main-light shadow result the trace kernel did not produce
 // (the two evaluate the same condition; a mismatch is an internal error).
 constexpr uint32_t ERR_SHADOW_MISMATCH = 8u;
+// A wait in the packet walk's queue ran out: the frame is incomplete.
+constexpr uint32_t ERR_QUEUE_WAIT = 16u;
 
 // Star binning of the fast path (sr_stars.cuh): tile side in pixels, and whether an observer's
 // stars are binned. The binning assumes a field of view within a 76-degree
