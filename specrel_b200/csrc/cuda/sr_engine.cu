@@ -662,6 +662,14 @@ sr_status sr_test_queued(sr_ctx* ctx, uint32_t queued[2]) {
     return SR_OK;
 }
 
+sr_status sr_test_star_room(sr_ctx* ctx, uint32_t entries) {
+    if (!ctx) return SR_ERR_INVALID_ARGUMENT;
+    CK(cudaStreamSynchronize(ctx->stream), "synchronize");
+    fast_release(ctx->fast);  // the graphs hold the room
+    ctx->fast.star_room = entries;
+    return SR_OK;
+}
+
 sr_status sr_render(sr_ctx* ctx, uint32_t idx, const SrGpuUniforms* u, uint32_t* fb, uint64_t fb_len, SrTimings* t) {
     if (!ctx || !u || !fb) return SR_ERR_INVALID_ARGUMENT;
     if (fb_len != (uint64_t)u->size[0] * u->size[1])

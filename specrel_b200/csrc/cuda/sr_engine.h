@@ -109,8 +109,10 @@ sr_status check_build_desc(sr_ctx* ctx, const SrBuildDesc* d, const SrGpuAttr* h
 }  // namespace sre
 
 // For this library's tests only (not part of the interface): the limit of a wait in the packet walk's queue
-// (FastCtx::fan_polls), and how many parts the two launches of the context's last frame queued.
+// (FastCtx::fan_polls), how many parts the two launches of the context's last frame queued, and the room of the
+// star lists per observer (FastCtx::star_room).
 extern "C" {
 sr_status sr_test_queue_polls(sr_ctx* ctx, uint32_t polls);
 sr_status sr_test_queued(sr_ctx* ctx, uint32_t queued[2]);
+sr_status sr_test_star_room(sr_ctx* ctx, uint32_t entries);
 }

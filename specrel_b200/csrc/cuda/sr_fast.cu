@@ -1701,7 +1701,9 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     }
     const size_t old_star = c.star_r.bytes + c.star_box.bytes + c.star_count.bytes + c.star_list.bytes + c.star_scan.bytes;
     // Star lists: room for every (observer, star) in 8 tiles; tiles past the room sum every star.
-    const uint32_t list_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(8ull * n * sd.num_stars, 1u << 20), 1u << 30);
+    const uint32_t list_cap = (uint32_t)std::min<uint64_t>(
+        c.star_room ? (uint64_t)c.star_room * n : std::max<uint64_t>(8ull * n * sd.num_stars, 1u << 20), 1u << 30);
+    c.batch_list_cap = list_cap;
     size_t scan_bytes = 0;
     if (binned) {
         const size_t pairs = (size_t)n * sd.num_stars;
@@ -2015,7 +2017,8 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     for (uint32_t k = 0; k <= level; ++k) loff[k + 1] = loff[k] + (size_t)lw[k] * lh[k];
     const size_t npx = (size_t)W * H;
     const uint32_t rblocks = (uint32_t)((npx + 255) / 256);
-    const size_t list_cap = stars_on ? c.star_list.bytes / 4 : 0;
+    // The forward pass's: the buffer may be larger from a batch of more observers, its entries beyond unwritten.
+    const size_t list_cap = stars_on ? c.batch_list_cap : 0;
     if ((e = c.adj_cam.ensure(sizeof(DCam))) != cudaSuccess) return e;
     if ((e = c.adj_partials.ensure((size_t)std::max(tiles, rblocks) * ADJ_SLOTS * sizeof(double))) != cudaSuccess) return e;
     if ((e = c.adj_out.ensure(2 * ADJ_SLOTS * sizeof(double))) != cudaSuccess) return e;

@@ -124,6 +124,8 @@ struct FastCtx {
     int staging_next = 0;
     const SrGpuUniforms* batch_U = nullptr;  // the last batch's, on the device
     const ObsDev* batch_obs = nullptr;
+    uint32_t batch_list_cap = 0;  // the last batch's room for star list entries
+    uint32_t star_room = 0;       // room per observer where not 0 (tests), else by the number of stars
     ~FastCtx() { for (cudaEvent_t e : staged) if (e) cudaEventDestroy(e); }
     std::map<uint64_t, GraphEntry> graphs;
 };
