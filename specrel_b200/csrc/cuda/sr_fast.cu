@@ -1980,6 +1980,33 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
 // ---------------------------------------------------------------------------------------------
 // The gradient of the image loss (sr_adjoint.cuh).
 // ---------------------------------------------------------------------------------------------
+// Whether kernels on the current device can read `bytes` at `p` as float4: aligned, memory of this device, and all
+// of it within one allocation.
+static bool readable_here(const void* p, size_t bytes) {
+    typedef int (*RangeFn)(unsigned long long*, size_t*, unsigned long long);  // cuMemGetAddressRange
+    static const RangeFn range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<RangeFn>(f);
+    }();
+    const unsigned long long at = reinterpret_cast<unsigned long long>(p);
+    cudaPointerAttributes a{};
+    int dev = 0;
+    unsigned long long base = 0;
+    size_t size = 0;
+    if (at % 16 != 0 || !range || cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == dev && range(&base, &size, at) == 0 && at - base <= size &&
+           bytes <= size - (at - base);
+}
+
 cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd, const double anchor[4],
                          const BBConst& bb, uint32_t* counters, const SrGpuUniforms& u, const SrCameraF64& cam,
                          const float* target, uint32_t level, bool frozen, uint32_t row0, uint32_t row1,
@@ -1991,19 +2018,8 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
             c.adj_r0 != row0 || c.adj_r1 != row1)
             return cudaErrorInvalidValue;
     } else {
-        // The forward frame: hits, shadow results, star lists and the HDR image the loss compares.
-        BatchRequest br{};
-        br.n = 1;
-        br.u = &u;
-        br.cam64 = &cam;
-        br.use_graph = true;
-        br.no_image = true;
         c.adj_valid = false;
-        if ((e = fast_render_batch(c, s, t, sd, anchor, bb, counters, br, st)) != cudaSuccess) return e;
     }
-    const uint32_t tx16 = (W + STAR_TILE - 1) / STAR_TILE, ty16 = (H + STAR_TILE - 1) / STAR_TILE;
-    const uint32_t tiles = tx16 * ty16;
-    const bool stars_on = sd.num_stars > 0 && stars_binned_for(u, sd.num_stars);
     // Pyramid geometry of the loss levels 0..level.
     uint32_t lw[8], lh[8];
     size_t loff[9];
@@ -2016,13 +2032,36 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     }
     for (uint32_t k = 0; k <= level; ++k) loff[k + 1] = loff[k] + (size_t)lw[k] * lh[k];
     const size_t npx = (size_t)W * H;
+    if ((e = c.adj_pyr.ensure(2 * loff[level + 1] * sizeof(float4))) != cudaSuccess) return e;
+    float4* pyr = c.adj_pyr.as<float4>();  // image levels 0..level
+    float4* tpyr = pyr + loff[level + 1];  // target levels 0..level
+    // The target is the caller's. Kernels read it where it lies when they can; else it is copied, which takes any
+    // float address and refuses memory that is not there. Copied always, a gradient took 550 against 546 us
+    // (320x200, level 3) and 839 against 829 (1280x800, level 0).
+    const float4* tgt0 = reinterpret_cast<const float4*>(target);
+    if (!readable_here(target, npx * sizeof(float4))) {
+        if ((e = cudaMemcpyAsync(tpyr, target, npx * sizeof(float4), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
+        tgt0 = tpyr;
+    }
+    if (!frozen) {
+        // The forward frame: hits, shadow results, star lists and the HDR image the loss compares.
+        BatchRequest br{};
+        br.n = 1;
+        br.u = &u;
+        br.cam64 = &cam;
+        br.use_graph = true;
+        br.no_image = true;
+        if ((e = fast_render_batch(c, s, t, sd, anchor, bb, counters, br, st)) != cudaSuccess) return e;
+    }
+    const uint32_t tx16 = (W + STAR_TILE - 1) / STAR_TILE, ty16 = (H + STAR_TILE - 1) / STAR_TILE;
+    const uint32_t tiles = tx16 * ty16;
+    const bool stars_on = sd.num_stars > 0 && stars_binned_for(u, sd.num_stars);
     const uint32_t rblocks = (uint32_t)((npx + 255) / 256);
     // The forward pass's: the buffer may be larger from a batch of more observers, its entries beyond unwritten.
     const size_t list_cap = stars_on ? c.batch_list_cap : 0;
     if ((e = c.adj_cam.ensure(sizeof(DCam))) != cudaSuccess) return e;
     if ((e = c.adj_partials.ensure((size_t)std::max(tiles, rblocks) * ADJ_SLOTS * sizeof(double))) != cudaSuccess) return e;
     if ((e = c.adj_out.ensure(2 * ADJ_SLOTS * sizeof(double))) != cudaSuccess) return e;
-    if ((e = c.adj_pyr.ensure(2 * loff[level + 1] * sizeof(float4))) != cudaSuccess) return e;
     if ((e = c.adj_weight.ensure(2 * npx * 3 * sizeof(double))) != cudaSuccess) return e;
     if ((e = c.adj_grid.ensure(npx)) != cudaSuccess) return e;
     if ((e = c.adj_hdr.ensure(npx * sizeof(float4))) != cudaSuccess) return e;
@@ -2030,8 +2069,6 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
     if (stars_on && (e = c.adj_star_sum.ensure(npx * ADJ_SUM * sizeof(float))) != cudaSuccess) return e;
     if (stars_on && (e = c.adj_star_n.ensure(npx * 4)) != cudaSuccess) return e;
     if (stars_on && (e = c.adj_pass.ensure(list_cap * 32)) != cudaSuccess) return e;
-    float4* pyr = c.adj_pyr.as<float4>();  // image levels 0..level
-    float4* tpyr = pyr + loff[level + 1];  // target levels 0..level
     double* g0 = c.adj_weight.as<double>();
     double* g1 = g0 + npx * 3;
     const dim3 b2(16, 16);
@@ -2041,7 +2078,6 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
         // Level 0 is the image and the target themselves.
         auto at = [&](const float4* level0, float4* levels, uint32_t k) { return k ? (const float4*)(levels + loff[k]) : level0; };
         const float4* img0 = reinterpret_cast<const float4*>(image);
-        const float4* tgt0 = reinterpret_cast<const float4*>(target);
         for (uint32_t k = 1; k <= level; ++k) {
             const dim3 g2((lw[k] + 15) / 16, (lh[k] + 15) / 16, 2);
             k_adj_down<<<g2, b2, 0, st>>>(at(img0, pyr, k - 1), at(tgt0, tpyr, k - 1), lw[k - 1], lh[k - 1], pyr + loff[k],

@@ -1,4 +1,5 @@
-"""What a gradient call (sr_adjoint) reads: the forward frame's star lists up to the room that frame had."""
+"""What a gradient call (sr_adjoint) reads: the forward frame's star lists up to the room that frame had, and the
+caller's target image wherever it lies."""
 import ctypes as C
 
 import numpy as np
@@ -59,3 +60,25 @@ def test_lists_longer_than_their_room_after_a_larger_batch(scene, room):
     finally:
         fresh.close()
         used.close()
+
+
+@pytest.mark.parametrize("level", [0, 3])
+def test_target_at_any_float_address(scene, level):
+    """The target is width * height * 4 floats: a view that starts at an odd float gives the same loss and
+    gradient, frozen evaluations too."""
+    u, cam = _uniforms(scene), sr.cam64(AT, FROM)
+    eng = _engine(scene)
+    try:
+        target = _target(eng, scene)
+        ref = _values(eng.adjoint(0, u, cam, target.data_ptr(), level=level))
+        frozen = eng.adjoint(0, u, cam, target.data_ptr(), level=level, frozen=True).loss
+        room = torch.zeros(4 * W * H + 8, device="cuda")
+        for shift in (1, 2, 3, 5):
+            view = room[shift:shift + 4 * W * H]
+            view.copy_(target.reshape(-1))
+            assert view.data_ptr() % 16 != 0
+            assert _values(eng.adjoint(0, u, cam, view.data_ptr(), level=level)) == ref
+            assert eng.adjoint(0, u, cam, view.data_ptr(), level=level, frozen=True).loss == frozen
+        assert _values(eng.adjoint(0, u, cam, target.data_ptr(), level=level)) == ref
+    finally:
+        eng.close()
