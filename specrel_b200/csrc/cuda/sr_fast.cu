@@ -125,9 +125,8 @@ __global__ void k_wide_fill(const SrGpuNode* nodes, uint32_t n, const uint32_t* 
 }
 
 // The packet walk's counters, a line each for those that many warps change.
-// FAN_LIST_HEAD: words of fan_list before its entries, the first of them `dirty`.
-constexpr uint32_t FAN_LIST_HEAD = 32;
-enum { FAN_NEXT = 0, FAN_HEAD = 32, FAN_TAIL = 64, FAN_FINISHED = 96, FAN_FIRST_DONE = 97, FAN_COUNTERS = 128 };
+// FAN_DIRTY: the word of FastCtx::sched that outlives a launch (the list holds entries), the others are cleared.
+enum { FAN_NEXT = 0, FAN_HEAD = 32, FAN_TAIL = 64, FAN_FINISHED = 96, FAN_FIRST_DONE = 97, FAN_COUNTERS = 128, FAN_DIRTY = 2 * FAN_COUNTERS + 1 };
 
 static cudaError_t lean_kernel_attrs(int max_smem);
 static cudaError_t fan_resident(int threads, int* blocks);
@@ -304,19 +303,20 @@ __device__ __forceinline__ Cam cam_of(const float4* cam, uint32_t o) {
 }
 
 // The observers of a batch; also clears the batch's counters (no launch of their own), and the packet walk's
-// queue where a wait that ran out in an earlier batch left entries in it (fan_dirty, null: no queue yet).
+// queue where a wait that ran out in an earlier batch left entries in it.
 __global__ void k_camera_batch(uint32_t n, const SrGpuUniforms* U, const SrCameraF64* cam64, const ObsDev* obs,
                                double a0, double a1, double a2, double a3, float4* cam, uint32_t* counters,
-                               uint32_t num_counters, uint32_t* sched, uint32_t num_sched, uint32_t* fan_dirty,
-                               uint32_t* fan_list, size_t num_fan_list) {
+                               uint32_t num_counters, uint32_t* sched, uint32_t num_sched, uint32_t* fan_list,
+                               size_t num_fan_list) {
     uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x == 0 && fan_dirty && *fan_dirty) {
+    if (blockIdx.x == 0 && sched[FAN_DIRTY]) {
         for (size_t k = threadIdx.x; k < num_fan_list; k += blockDim.x) fan_list[k] = 0u;
         __syncthreads();
-        if (threadIdx.x == 0) *fan_dirty = 0u;
+        if (threadIdx.x == 0) sched[FAN_DIRTY] = 0u;
     }
     for (uint32_t k = o; k < num_counters; k += gridDim.x * blockDim.x) counters[k] = 0u;
-    for (uint32_t k = o; k < num_sched; k += gridDim.x * blockDim.x) sched[k] = 0u;
+    for (uint32_t k = o; k < num_sched; k += gridDim.x * blockDim.x)
+        if (k != FAN_DIRTY) sched[k] = 0u;
     if (o >= n) return;
     float4* out = cam + 6ull * o;
     if (obs[o].has_cam64) {
@@ -1655,7 +1655,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         // Without room for the queue the rays walk alone. The queue's own buffer: its entries are zero
         // between launches, whatever the next one's size, the list's are not.
         packet = sh.total_tiles < FAN_MAX_TILES &&
-                 c.fan_list.ensure((FAN_LIST_HEAD + (size_t)sh.total_tiles * FAN_QUEUED_PER_TILE) * 4) == cudaSuccess &&
+                 c.fan_list.ensure((size_t)sh.total_tiles * FAN_QUEUED_PER_TILE * 4) == cudaSuccess &&
                  c.fan_shadows.ensure((size_t)sh.total_tiles * FAN_SHADOWS_PER_TILE * 4) == cudaSuccess;
         if (c.fan_list.bytes != old || c.fan_shadows.bytes != old_shadows) drop_graphs();
         if (c.fan_list.bytes != old && c.fan_list.p) {
@@ -1684,7 +1684,10 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     if ((e = c.slots.ensure((size_t)sh.total_px * 4)) != cudaSuccess) return e;
     if ((e = c.shadow.ensure((size_t)sh.total_px)) != cudaSuccess) return e;  // shadow states
     if ((e = c.hdr.ensure((size_t)sh.total_pyr * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = c.sched.ensure(std::max<size_t>((size_t)c.num_sms + 1, 2 * FAN_COUNTERS + 1) * 4)) != cudaSuccess) return e;
+    if (!c.sched.p) {
+        if ((e = c.sched.ensure(std::max<size_t>((size_t)c.num_sms + 1, FAN_DIRTY + 1) * 4)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(c.sched.p, 0, c.sched.bytes, st)) != cudaSuccess) return e;
+    }
     bool shadows = false;  // some observer casts shadow rays
     for (uint32_t i = 0; i < n; ++i)
         shadows = shadows || (r.u[i].mode == 0u && r.u[i].shadow_mode != 0u && r.u[i].num_flashes == 0u);
@@ -1759,8 +1762,7 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         k_camera_batch<<<(n + 63) / 64, 64, 0, st>>>(n, in.U, in.cam64, in.obs, anchor[0], anchor[1], anchor[2], anchor[3],
                                                      c.cam.as<float4>(), counters, r.count_work ? 16u : 4u,
                                                      c.sched.as<uint32_t>(), (uint32_t)(c.sched.bytes / 4),
-                                                     c.fan_list.as<uint32_t>(), c.fan_list.as<uint32_t>() + FAN_LIST_HEAD,
-                                                     c.fan_list.p ? c.fan_list.bytes / 4 - FAN_LIST_HEAD : 0);
+                                                     c.fan_list.as<uint32_t>(), c.fan_list.bytes / 4);
         if (timed) cudaEventRecord(r.ev[0], st);
         TraceBatchArgs ta;
         ta.top_n = 0;
@@ -1805,8 +1807,8 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
                 FanTasks ft;
                 ft.count = c.sched.as<uint32_t>();
                 ft.num_shadows = ft.count + 2 * FAN_COUNTERS;
-                ft.dirty = c.fan_list.as<uint32_t>();
-                ft.list = ft.dirty + FAN_LIST_HEAD;
+                ft.dirty = ft.count + FAN_DIRTY;
+                ft.list = c.fan_list.as<uint32_t>();
                 ft.lost = c.fan_lost.as<uint32_t>();
                 ft.polls = c.fan_polls;
                 ft.shadows = c.fan_shadows.as<uint32_t>();
