@@ -919,25 +919,29 @@ __device__ __forceinline__ uint32_t warp_next(uint32_t* counter) {
     if ((threadIdx.x & 31u) == 0) t = atomicAdd(counter, 1u);
     return __shfl_sync(FULL_WARP, t, 0);
 }
-// Puts a task (tile, part) for each lane that has one at the end of `list`.
+__device__ __forceinline__ void store_release(uint32_t* p, uint32_t v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// Puts a task (tile, part) for each lane that has one at the end of `list`, after all lanes' writes: the warp's
+// barrier orders them before each lane's releasing store.
 __device__ __forceinline__ void fan_list(uint32_t* list, uint32_t* tail, uint32_t tile, uint32_t part, bool has) {
     const uint32_t lane = threadIdx.x & 31u, which = __ballot_sync(FULL_WARP, has);
     uint32_t at = 0;
     if (lane == 0) at = atomicAdd(tail, (uint32_t)__popc(which));
     at = __shfl_sync(FULL_WARP, at, 0) + (uint32_t)__popc(which & ((1u << lane) - 1u));
-    if (has) *(volatile uint32_t*)(list + at) = (tile << FAN_PARTS_LOG) + part + 1u;
-}
-// The same into the queue, after this warp's writes.
-__device__ __forceinline__ void fan_push(const FanTasks& q, uint32_t tile, uint32_t part, bool has) {
-    __threadfence();
     __syncwarp();
+    if (has) store_release(list + at, (tile << FAN_PARTS_LOG) + part + 1u);
+}
+__device__ __forceinline__ void fan_push(const FanTasks& q, uint32_t tile, uint32_t part, bool has) {
     fan_list(q.list, q.count + FAN_TAIL, tile, part, has);
 }
 // A warp's first tasks are done: `mine` of them.
 __device__ __forceinline__ void fan_first_done(const FanTasks& q, uint32_t mine) {
-    __threadfence();
     __syncwarp();
-    if ((threadIdx.x & 31u) == 0 && mine) atomicAdd(q.count + FAN_FIRST_DONE, mine);
+    if ((threadIdx.x & 31u) == 0 && mine) {
+        __threadfence();
+        atomicAdd(q.count + FAN_FIRST_DONE, mine);
+    }
 }
 __device__ __forceinline__ void fan_finished(const FanTasks& q) {
     __syncwarp();
@@ -982,6 +986,8 @@ __device__ __forceinline__ uint32_t fan_take(const FanTasks& q, uint32_t first, 
             entry = 0;
         }
     }
+    // Lane 0 acquired the entry; the barrier orders the other lanes' reads of what its task left behind it.
+    __syncwarp();
     return __shfl_sync(FULL_WARP, entry, 0);
 }
 
