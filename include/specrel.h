@@ -402,7 +402,9 @@ sr_status sr_render_batch(sr_ctx* ctx, uint32_t scene_idx, const SrGpuUniforms* 
  * anchor it is the f32 origin) and runs along `dir` over (t_min, t_max). `hits` receives, per ray,
  * the hit simplex (the caller's index through leaf_to_orig, else the leaf slot; 0xFFFFFFFF on a
  * miss), its parameter lambda, the interpolated proper time, the event (the anchor added back in
- * double), the tetrahedron barycentrics, the uv and the material. Host buffers; blocking. */
+ * double), the tetrahedron barycentrics, the uv and the material. Where leaves' boxes hold their
+ * records the hit is the reference traversal's; in an uploaded tree whose do not, a record hit more than
+ * 0.1% in lambda before its leaf's box is entered may lose to one behind it. Host buffers; blocking. */
 typedef struct SrRay {
     double origin[4];  /* (t, x, y, z) */
     float dir[4];
@@ -535,7 +537,8 @@ typedef struct SrTuning {
                                  parameter (the records' 1e-4 box padding keeps a margin of
                                  1e-4 / |d| in ray parameter against its rounding); with
                                  stack_smem 0, top_levels 0 and the single-tile schedule. Launches
-                                 too small to gain by it take the per-ray order all the same.
+                                 too small to gain by it take the per-ray order all the same, and so
+                                 do trees with a box that does not hold its children's.
                                  0: each ray walks the tree in its own near-first order (work
                                  counts, SR_FLAG_COUNT_WORK, always come from this order) */
 } SrTuning;

@@ -29,20 +29,27 @@ constexpr int FAN_RAYS = 2;             // rays per lane of a closest-hit walk
 // five levels from the root leaves whatever remains there.
 // ---------------------------------------------------------------------------------------------
 struct FanCounts {
-    uint32_t fans, conflict, root_total;
+    uint32_t fans, root_total;
+    uint32_t conflict;                       // a child claimed twice, or a box that does not hold its children's
     uint32_t units[FAN_LEVELS + 2];          // per level
     uint32_t reached[FAST_MAX_DEPTH + 2];    // nodes per depth (the marking)
 };
 
 // parent[child] = i for both children of every internal node (of every reached node, when `reach` is
-// given). Free room of an arena holds stale nodes whose links may point into the live tree: a child
-// claimed twice sets `conflict`, and the build marks what the root reaches first.
+// given). A child claimed twice sets `conflict`, and so does a box that does not hold its children's: a fan node
+// leaves out the boxes between it and its entries, which only hides nothing from a ray where boxes are nested
+// (as every builder here makes them; an uploaded tree need not). Free room of an arena holds stale nodes whose
+// links may point into the live tree: on a conflict the build marks what the root reaches and looks again.
 __global__ void k_fan_parents(const SrGpuNode* nodes, uint32_t n, const uint32_t* reach, uint32_t* parent, FanCounts* fc) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || nodes[i].count != 0 || (reach && !reach[i])) return;
     const uint32_t c[2] = {nodes[i].left, nodes[i].right_or_first};
-    for (int k = 0; k < 2; ++k)
-        if (c[k] >= n || c[k] == 0 || atomicExch(parent + c[k], i) != FAN_NONE) fc->conflict = 1;
+    for (int k = 0; k < 2; ++k) {
+        bool sound = c[k] < n && c[k] != 0 && atomicExch(parent + c[k], i) == FAN_NONE;
+        for (int a = 0; a < 4 && sound; ++a)  // false for a NaN
+            sound = nodes[c[k]].min[a] >= nodes[i].min[a] && nodes[c[k]].max[a] <= nodes[i].max[a];
+        if (!sound) fc->conflict = 1;
+    }
 }
 
 // One level of the breadth-first marking: the nodes of depth `level`, which lie in the queue behind those of
@@ -152,8 +159,8 @@ __global__ void __launch_bounds__(128) k_fan_fill(const SrGpuNode* nodes, uint32
     ref[(size_t)w * 32u + lane] = r;
 }
 
-// Builds the layout (s.fan_*); s.fan_levels stays 0 where there is none: memory short, or a tree
-// that needs more than FAN_LEVELS levels. `scratch`: 6 n + 1024 words.
+// Builds the layout (s.fan_*); s.fan_levels stays 0 where there is none: memory short, a tree that needs more than
+// FAN_LEVELS levels, or boxes that are not nested. `scratch`: 6 n + 1024 words.
 static cudaError_t fan_build(FastScene& s, const SrGpuNode* nodes, uint32_t n, uint32_t* scratch, cudaStream_t st) {
     s.fan_levels = 0;
     uint32_t *parent = scratch, *acc = parent + n, *total = acc + n, *uref = total + n, *units = uref + n, *roots = units + n;
@@ -163,7 +170,7 @@ static cudaError_t fan_build(FastScene& s, const SrGpuNode* nodes, uint32_t n, u
     const uint32_t* reach = nullptr;
     cudaError_t e;
     auto look = [&]() -> cudaError_t {
-        cudaError_t x = cudaMemcpyAsync(&h, fc, 12, cudaMemcpyDeviceToHost, st);
+        cudaError_t x = cudaMemcpyAsync(&h, fc, offsetof(FanCounts, units), cudaMemcpyDeviceToHost, st);
         return x == cudaSuccess ? cudaStreamSynchronize(st) : x;
     };
     if ((e = cudaMemsetAsync(parent, 0xFF, (size_t)n * 4, st)) != cudaSuccess) return e;
@@ -194,7 +201,7 @@ static cudaError_t fan_build(FastScene& s, const SrGpuNode* nodes, uint32_t n, u
         ++levels;
         if (levels < usual && levels < FAN_LEVELS) continue;
         if ((e = look()) != cudaSuccess) return e;
-        if (h.conflict) return cudaSuccess;  // not a tree: no fan layout
+        if (h.conflict) return cudaSuccess;  // not a tree of nested boxes: no fan layout
     } while (h.root_total == 0 && levels < FAN_LEVELS);
     if (h.root_total == 0) return cudaSuccess;
     if (s.fan_box.ensure_grow((size_t)h.fans * 64 * sizeof(float4)) != cudaSuccess ||

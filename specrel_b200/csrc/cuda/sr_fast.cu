@@ -18,6 +18,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 
 #include "sr_camera.cuh"
