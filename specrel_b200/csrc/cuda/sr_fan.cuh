@@ -497,7 +497,7 @@ __device__ __forceinline__ void fan_bounds(const SrGpuUniforms& U, const Cam& ca
     const uint32_t sx = (1u << w_log) - 1u, sy = (1u << h_log) - 1u;
     const float kx = __fdividef(2.0f * U.half_wh[0], (float)U.size[0]), ky = __fdividef(-2.0f * U.half_wh[1], (float)U.size[1]);
     const float c0 = U.slice_mode == 0u ? -1.0f : (U.slice_mode == 2u ? 1.0f : 0.0f);
-    const float slack = (6e-6f + 2e-6f * (U.half_wh[0] + U.half_wh[1])) * fmaxf(max3f(max_b(cam.e0), max_b(cam.e1), max_b(cam.e2)), max_b(cam.e3));
+    const float slack = (6e-6f + 2e-6f * (fabsf(U.half_wh[0]) + fabsf(U.half_wh[1]))) * fmaxf(max3f(max_b(cam.e0), max_b(cam.e1), max_b(cam.e2)), max_b(cam.e3));
     float4 d[FAN_RAYS];
     const float ix = sx ? __fdividef(2.0f, (float)sx) : 0.0f, iy = sy ? __fdividef(2.0f, (float)sy) : 0.0f;
 #pragma unroll
