@@ -326,7 +326,9 @@ __device__ __forceinline__ void fan_interval(float4 bmin, float4 bmax, float4 no
 // largest value over the rays is its value at `mid` plus the magnitudes along du, dv and the rest. The
 // same for v, w and 1 - u - v - w. What a float test can differ by from these is bounded by
 // 2^-18 |B|_1 |n|_1 D (|o| + |v0 - o| + lambda D), D the largest direction component: the products and
-// sums of the test and of this function round at 2^-24 of such terms at most 36 times.
+// sums of the test and of this function round at 2^-24 of such terms at most 36 times. Every comparison rejects
+// only where it holds: a record with a NaN or an infinity goes on to the rays' own tests, whose comparisons a NaN
+// passes likewise.
 __device__ __forceinline__ bool fan_record(const float4* g, const FanRays& f, float t_max, float* lam) {
     const float4 n = __ldg(g + 1), v0 = __ldg(g), B1 = __ldg(g + 2), B2 = __ldg(g + 3), B3 = __ldg(g + 4);
     const float4 mid = f.mid, du = f.du, dv = f.dv, no = f.no;
@@ -350,7 +352,7 @@ __device__ __forceinline__ bool fan_record(const float4* g, const FanRays& f, fl
     if (!edge) *lam = lo;
     const float hi = fminf(__fdividef(num + num_err, den_lo) * 1.0001f, t_max);
     const float err = 3.8147e-6f * n1 * d_max * (f.o_max + w_max + hi * d_max);
-    bool may = num >= -num_err && lo < t_max;  // not behind the rays, nor beyond their hits
+    bool may = !(num < -num_err) && !(lo >= t_max);  // not behind the rays, nor beyond their hits
     float us = 0.0f, bc = 0.0f, bu = 0.0f, bv = 0.0f, b1 = 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -358,7 +360,7 @@ __device__ __forceinline__ bool fan_record(const float4* g, const FanRays& f, fl
         const float U = 1e-5f - dot_b(B, w), c = dot_b(B, mid), u = dot_b(B, du), v = dot_b(B, dv), l1 = l1_b(B);
         const float top = fmaf(U, nc, num * c) + fabsf(fmaf(U, nu, num * u)) + fabsf(fmaf(U, nv, num * v)) +
                           fmaf(fabsf(U), nr, fmaf(fabsf(num), res, err) * l1);
-        may = may && top >= 0.0f;
+        may = may && !(top < 0.0f);
         us += U;
         bc += c;
         bu += u;
@@ -368,7 +370,7 @@ __device__ __forceinline__ bool fan_record(const float4* g, const FanRays& f, fl
     const float S = 1.00005f - us;  // 1 + 1e-5 - u - v - w (each U carries 1e-5), and the rounding of the three sums
     const float top = fmaf(S, nc, -num * bc) + fabsf(fmaf(S, nu, -num * bu)) + fabsf(fmaf(S, nv, -num * bv)) +
                       fmaf(fabsf(S), nr, fmaf(fabsf(num), res, err) * b1);
-    return edge || (may && top >= 0.0f);
+    return edge || (may && !(top < 0.0f));
 }
 
 // A quantity that is affine over the rays up to a remainder: c + a u + b v + e, |a|, |b| <= 1, |e| <= r.
@@ -423,7 +425,7 @@ __device__ __forceinline__ bool fan_record_any(const float4* g, const FanShadows
         const float l1 = l1_b(B);
         const FanAff U{1e-5f - dot_b(B, w), dot_b(B, f.ou), dot_b(B, f.ov), dot_b(ab, f.ores)};
         const FanAff E{dot_b(B, f.mid), dot_b(B, f.du), dot_b(B, f.dv), dot_b(ab, f.res)};
-        may = may && aff_top2(U, den, num, E) >= -err * l1;
+        may = may && !(aff_top2(U, den, num, E) < -err * l1);
         us.c += U.c;
         us.u += U.u;
         us.v += U.v;
@@ -440,7 +442,7 @@ __device__ __forceinline__ bool fan_record_any(const float4* g, const FanShadows
     bs.c = -bs.c;
     bs.u = -bs.u;
     bs.v = -bs.v;
-    return may && aff_top2(us, den, num, bs) >= -err * b1;
+    return may && !(aff_top2(us, den, num, bs) < -err * b1);
 }
 
 // The records of the leaves `leaves` (lanes holding their references) and of the leaf in progress, dealt

@@ -1588,7 +1588,7 @@ __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const 
                 const bool h = lane < held && intersect_lean(ws.geoms + 5u * mine, no, d, r.t_min,
                                                              __uint_as_float(__float_as_uint(t_max) + 1u), &gh);
                 if (!__any_sync(FULL_WARP, h)) continue;
-                if (__any_sync(FULL_WARP, h && gh.lambda < entry)) reference = true;
+                if (__any_sync(FULL_WARP, h && !(gh.lambda >= entry))) reference = true;  // a NaN too
                 const uint32_t nearest = redux_min(h ? __float_as_uint(gh.lambda) : FAN_NONE);
                 for (uint32_t m = __ballot_sync(FULL_WARP, h && __float_as_uint(gh.lambda) == nearest); m; m &= m - 1u) {
                     const uint32_t c = (uint32_t)__ffs((int)m) - 1u, rec = __shfl_sync(FULL_WARP, mine, c);

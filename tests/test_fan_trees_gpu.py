@@ -1,5 +1,6 @@
-"""The fan layout (sr_fan.cuh) leaves boxes of the tree out, which a ray does not notice where boxes are nested. An
-uploaded tree need not be: its frames and caller rays must still be the reference's walk over every box."""
+"""The fan layout (sr_fan.cuh) on what an upload may hold. It leaves boxes of the tree out, which a ray does not
+notice where boxes are nested: where they are not, frames and caller rays must still be the reference's walk over
+every box. Records may hold NaNs and infinities, which pass the ray test's comparisons."""
 import numpy as np
 import pytest
 
@@ -61,3 +62,53 @@ def test_caller_rays_into_such_a_tree(engine, shrink):
     a, b = engine.trace_rays(IDX, rays), engine.trace_rays(IDX, far)
     assert (a["slot"] == b["slot"]).all() and (a["lambda_"] == b["lambda_"] * np.float32(UP)).all()
     assert (a["slot"] != 0xFFFFFFFF).any()
+
+
+def _broken(row, value):
+    """Every seventh record with a row of its barycentric matrix set to `value`; hit ids are leaf slots."""
+    p = _tree(False)
+    geoms = p.geoms.copy()
+    geoms.view(np.float32).reshape(-1, 5, 4)[::7, row] = value
+    return sr.PackedScene(p.nodes, geoms, p.attrs, p.materials, p.stars, 0, p.light_pos, None)
+
+
+def _early(packed, u, pixels, slots, lam):
+    """Whether a hit lies before the entry of its leaf's box, where the packet's order need not be the reference's
+    (SrTuning.packet's condition); by the ray and the box in 64 bits, up to a rounding of 1e-5."""
+    leaf = np.flatnonzero(packed.nodes["count"] > 0)
+    leaf = leaf[np.argsort(packed.nodes["right_or_first"][leaf])]
+    first = packed.nodes["right_or_first"][leaf]
+    w, h = u.size[0], u.size[1]
+    e = np.array([list(r) for r in u.e])
+    out = np.zeros(len(pixels), bool)
+    for k, (pix, slot, la) in enumerate(zip(pixels, slots, lam)):
+        if slot == 0xFFFFFFFF:
+            continue
+        n = np.array([(2.0 * (pix % w + 0.5) / w - 1.0) * u.half_wh[0], (1.0 - 2.0 * (pix // w + 0.5) / h) * u.half_wh[1], 1.0])
+        n /= np.linalg.norm(n)
+        d = -e[0] + n[0] * e[1] + n[1] * e[2] + n[2] * e[3]
+        node = packed.nodes[leaf[np.searchsorted(first, slot, "right") - 1]]
+        a, b = (node["min"] - np.array(list(u.cam_pos))) / d, (node["max"] - np.array(list(u.cam_pos))) / d
+        out[k] = la < np.minimum(a, b).max() * (1.0 + 1e-5)
+    return out
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("row", [2, 3, 4])
+def test_records_with_nans_and_infinities(engine, row, value):
+    """Such a record is hit over more of its hyperplane than its tetrahedron. Pixels may differ from the reference's
+    only where one of the two hits lies before its leaf's box is entered."""
+    packed = _broken(row, value)
+    engine.upload(IDX, packed)
+    hits = broken = 0
+    for pos in ((0.0, 0.0, 0.0, 0.0), (-20.0, 5.0, 3.0, -4.0)):
+        u = sr.uniforms(sr.camera(pos, 110.0, rapidity=(0.4, 0.1, -0.3)), 640, 400, 0, 0, 0,
+                        num_nodes=len(packed.nodes), light_pos=packed.light_pos)
+        fast, plain = (engine.render(IDX, u, path=path, aux=True) for path in (sr.SR_PATH_FAST, sr.SR_PATH_PLAIN))
+        diff = np.flatnonzero(fast.hit_id != plain.hit_id)
+        early = _early(packed, u, diff, fast.hit_id[diff], fast.lam[diff]) | _early(packed, u, diff, plain.hit_id[diff], plain.lam[diff])
+        assert early.all()
+        hit = plain.hit_id != 0xFFFFFFFF
+        hits += int(hit.sum())
+        broken += int((hit & (plain.hit_id % 7 == 0)).sum())
+    assert broken > hits / 10  # they are met often
