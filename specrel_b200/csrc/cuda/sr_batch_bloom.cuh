@@ -70,9 +70,12 @@ __global__ void k_bloom_up_batch(float4* hdr, const ObsDev* obs, const uint32_t*
 }
 
 // The coarse levels of every observer, one block each: down to levels k0..6, then level k += up(level k + 1) for
-// 5..k0. A level of at most BLOOM_TAIL pixels keeps a block a few microseconds; as launches of their own the
-// eight passes from level 3 on took 4 us each whatever their size (12 launches and 53 us for a 320x200 frame).
-constexpr uint32_t BLOOM_TAIL = 20000;
+// 5..k0. The levels of at most BLOOM_TAIL pixels, a pixel per thread: such a pass costs a block less than a launch
+// of its own, and each further round of 1024 pixels as much again, on one SM. Frames in turn by the largest level
+// taken (us; none, 1100, 4200 and 20000 pixels): 320x200 160, 156, 162, 205; 471x163 121, 119, 119, 182; 8 of
+// 1280x800 593, 588, 590, 639; 64 of 320x200 579, 558, 558, 577; the bloom alone 58, 37, 40, 79 at 320x200 and
+// 193, 187, 188, 231 for the eight.
+constexpr uint32_t BLOOM_TAIL = 1024;
 __global__ void __launch_bounds__(1024) k_bloom_tail_batch(float4* hdr, const ObsDev* obs, int k0) {
     const ObsDev& od = obs[blockIdx.x];
     for (int k = k0; k <= SR_BLOOM_LEVELS; ++k) {
