@@ -159,7 +159,7 @@ namespace {
 // call has read (frames that stay on the device): reported once.
 sr_status queue_errors(sr_ctx* ctx, uint32_t flags) {
     volatile uint32_t* lost = ctx->fast.fan_lost.as<uint32_t>();
-    if (!(flags & ERR_QUEUE_WAIT) && !*lost) return SR_OK;
+    if (!lost || (!(flags & ERR_QUEUE_WAIT) && !*lost)) return SR_OK;  // null: no packet frame yet
     *lost = 0;
     return fail(ctx, SR_ERR_CUDA, "internal error: a wait in the trace kernel's queue ran out, a frame is incomplete");
 }

@@ -148,9 +148,6 @@ cudaError_t fast_init(FastCtx& c, const cudaDeviceProp& prop) {
         if (e != cudaSuccess) return e;
         c.fan_blocks[threads / 128] = (uint32_t)std::max(n, 1);
     }
-    cudaError_t e = c.fan_lost.ensure(64);
-    if (e != cudaSuccess) return e;
-    std::memset(c.fan_lost.p, 0, c.fan_lost.bytes);
     return lean_kernel_attrs(c.max_smem);
 }
 
@@ -1661,7 +1658,8 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
         const size_t old = c.fan_list.bytes, old_shadows = c.fan_shadows.bytes;
         // Without room for the queue the rays walk alone. The queue's own buffer: its entries are zero
         // between launches, whatever the next one's size, the list's are not.
-        packet = sh.total_tiles < FAN_MAX_TILES &&
+        if (!c.fan_lost.p && c.fan_lost.ensure(64) == cudaSuccess) std::memset(c.fan_lost.p, 0, c.fan_lost.bytes);
+        packet = sh.total_tiles < FAN_MAX_TILES && c.fan_lost.p &&
                  c.fan_list.ensure((size_t)sh.total_tiles * FAN_QUEUED_PER_TILE * 4) == cudaSuccess &&
                  c.fan_shadows.ensure((size_t)sh.total_tiles * FAN_SHADOWS_PER_TILE * 4) == cudaSuccess;
         if (c.fan_list.bytes != old || c.fan_shadows.bytes != old_shadows) drop_graphs();
