@@ -692,12 +692,12 @@ sr_status sr_trace_rays(sr_ctx* ctx, uint32_t idx, const SrRay* rays, uint32_t n
     DevBuf& din = n <= RAY_BUFFER_KEEP ? ctx->rays_in : own_in;
     DevBuf& dout = n <= RAY_BUFFER_KEEP ? ctx->rays_out : own_out;
     CK(din.ensure((size_t)n * sizeof(SrRay)), "ray buffer");
-    CK(dout.ensure((size_t)n * sizeof(SrRayHit)), "hit buffer");
+    CK(dout.ensure((size_t)n * (sizeof(SrRayHit) + sizeof(uint32_t))), "hit buffer");
     cudaStream_t sm = ctx->stream;
     CK(cudaMemcpyAsync(din.p, rays, (size_t)n * sizeof(SrRay), cudaMemcpyHostToDevice, sm), "rays in");
     CK(cudaMemsetAsync(ctx->counters.p, 0, 16, sm), "clear counters");
-    CK(fast_trace_rays(s.fast, scene_dev(ctx, s), s.anchor, din.as<SrRay>(), n, dout.as<SrRayHit>(), ctx->counters.as<uint32_t>(),
-                       sm),
+    CK(fast_trace_rays(s.fast, scene_dev(ctx, s), s.anchor, din.as<SrRay>(), n, dout.as<SrRayHit>(),
+                       reinterpret_cast<uint32_t*>(dout.as<SrRayHit>() + n), ctx->counters.as<uint32_t>(), sm),
        "ray kernel");
     CK(cudaMemcpyAsync(hits, dout.p, (size_t)n * sizeof(SrRayHit), cudaMemcpyDeviceToHost, sm), "hits out");
     uint32_t counters[4] = {0, 0, 0, 0};

@@ -1481,12 +1481,12 @@ static WideScene wide_scene(const FastScene& s, const SceneDev& sd) {
     return ws;
 }
 
-// Whether the node layouts give a ray trace_ref's hit bit for bit: their comparisons assume a positive range
-// and finite values (no product of a coordinate, an inverse direction and a box overflows to a NaN).
+// Whether the node layouts give a ray trace_ref's hit bit for bit: their comparisons assume a range from 0 or
+// beyond and finite values (no product of a coordinate, an inverse direction and a box overflows to a NaN).
 __device__ __forceinline__ bool layout_ray(float4 o, float4 d, float t_min, float t_max) {
     const float lim = 1e12f;
     const auto in = [&](float v) { return fabsf(v) <= lim; };  // false for a NaN
-    return t_min > 0.0f && t_max > 0.0f && in(o.x) && in(o.y) && in(o.z) && in(o.w) && in(d.x) && in(d.y) && in(d.z) && in(d.w);
+    return t_min >= 0.0f && t_max > 0.0f && in(o.x) && in(o.y) && in(o.z) && in(o.w) && in(d.x) && in(d.y) && in(d.z) && in(d.w);
 }
 
 __device__ __forceinline__ void write_ray_hit(const SceneDev& s, double a0, double a1, double a2, double a3, float4 o, float4 d,
@@ -1520,11 +1520,13 @@ __device__ __forceinline__ void write_ray_hit(const SceneDev& s, double a0, doub
     *to = out;
 }
 
-// Caller rays (sr_trace_rays), one thread per ray on the reference's nodes: scenes without the layouts.
+// Caller rays (sr_trace_rays), one thread per ray on the reference's nodes: scenes without the layouts, long lists,
+// and the rays that the walk over the fan layout leaves (`rest`, counters[2] of them; null: all n).
 __global__ void __launch_bounds__(64) k_trace_rays(const SceneDev s, double a0, double a1, double a2, double a3, const SrRay* rays,
-                                                   uint32_t n, SrRayHit* hits, uint32_t* counters) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+                                                   uint32_t n, const uint32_t* rest, SrRayHit* hits, uint32_t* counters) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (rest ? counters[2] : n)) return;
+    if (rest) i = rest[i];
     const SrRay r = rays[i];
     const float4 o = v4((float)(r.origin[0] - a0), (float)(r.origin[1] - a1), (float)(r.origin[2] - a2),
                         (float)(r.origin[3] - a3));
@@ -1542,13 +1544,14 @@ __global__ void __launch_bounds__(64) k_trace_rays(const SceneDev s, double a0, 
 // smallest lambda; when the box's entry parameter as computed is not beyond it, every box on the way to
 // k is entered before any hit so far (boxes hold their children's), so the reference tests k, and no
 // nearer one. A hit before its box's entry is rounding against the build's padding; boxes are culled only
-// 0.1% beyond the closest hit, so that one is met rather than culled, and the ray then takes the
-// reference's own walk. Of hits at equal lambda the reference keeps the one its order meets first
-// (packet_precedes).
+// 0.1% beyond the closest hit, so that one is met rather than culled, and the ray is then left to the
+// reference's own walk, a thread per ray (k_trace_rays, with the rays that the layouts do not take: with the whole
+// warp here, a list of them took up to 3 times as long). Of hits at equal lambda the reference keeps the one its
+// order meets first (packet_precedes).
 template <bool OCT>
 __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const __grid_constant__ WideScene ws, double a0, double a1,
-                                                        double a2, double a3, const SrRay* rays, uint32_t n, SrRayHit* hits,
-                                                        uint32_t* counters) {
+                                                        double a2, double a3, const SrRay* rays, uint32_t n, uint32_t* rest,
+                                                        SrRayHit* hits, uint32_t* counters) {
     const uint32_t i = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (i >= n) return;
     const SrRay r = rays[i];
@@ -1574,7 +1577,8 @@ __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const 
             uint32_t ref = __ldg(ws.fan_ref + (size_t)node * 32u + lane);
             slab_interval(__ldg(bx + lane), __ldg(bx + 32u + lane), no, inv, r.t_min, limit, &en, &ex);
             const bool meets = ex >= en, leaf = (ref & REF_LEAF) != 0u;
-            uint32_t key = meets && !leaf ? ((__float_as_uint(en) & ~31u) | lane) : FAN_NONE;
+            // en + 0: no sign bit on a zero entry.
+            uint32_t key = meets && !leaf ? ((__float_as_uint(en + 0.0f) & ~31u) | lane) : FAN_NONE;
             FanDeal deal{__ballot_sync(FULL_WARP, meets && leaf), 0u, 0u, 0u};
             while (deal.leaves | deal.left) {
                 uint32_t mine, from;
@@ -1614,22 +1618,33 @@ __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const 
             st[depth++] = make_uint2(key, ref);
         }
     }
-    if (reference) slot = trace_ref(s, o, d, r.t_min, r.t_max, &best, counters + 1);  // the same for every lane
-    if (lane == 0) write_ray_hit(s, a0, a1, a2, a3, o, d, slot, best, hits + i);
+    if (lane != 0) return;
+    if (reference) rest[atomicAdd(counters + 2, 1u)] = i;
+    else write_ray_hit(s, a0, a1, a2, a3, o, d, slot, best, hits + i);
 }
 
+// Lists longer than this walk a ray per thread: a warp per ray shortens the longest ray's chain of loads, which a
+// short list waits for, and issues more for each, which a long one waits for. Whole calls, thread against warp per ray
+// (us): 65,536 rays into 8 accelerated bodies 1362 and 817, into 64 of them 3429 and 1988 (neighbouring directions
+// 1842 and 1192), into 147k tetrahedra 867 and 844; 262,144: 2766 and 2700, 7193 and 7129 (3261 and 4310), 2297 and
+// 3105; a million: 12.7 and 13.5 ms, 29.5 and 30.8 (11.7 and 19.3), 11.2 and 14.9.
+constexpr uint32_t RAYS_LONG = 1u << 16;
+
 cudaError_t fast_trace_rays(const FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
-                            SrRayHit* hits, uint32_t* counters, cudaStream_t st) {
+                            SrRayHit* hits, uint32_t* rest, uint32_t* counters, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const WideScene ws = wide_scene(s, sd);
     const double *a = anchor;
     const uint32_t blocks = (n + 3) / 4;
-    if (!s.usable || s.fan_levels == 0)
-        k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, hits, counters);
-    else if (ws.oct_copies)
-        k_trace_rays_fan<true><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, hits, counters);
+    if (!s.usable || s.fan_levels == 0 || n > RAYS_LONG) {
+        k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, nullptr, hits, counters);
+        return cudaGetLastError();
+    }
+    if (ws.oct_copies)
+        k_trace_rays_fan<true><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
     else
-        k_trace_rays_fan<false><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, hits, counters);
+        k_trace_rays_fan<false><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
+    k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
     return cudaGetLastError();
 }
 

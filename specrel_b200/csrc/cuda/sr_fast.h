@@ -171,9 +171,10 @@ cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, cons
                          const BBConst& bb, uint32_t* counters, const SrGpuUniforms& u, const SrCameraF64& cam,
                          const float* target, uint32_t level, bool frozen, uint32_t row0, uint32_t row1,
                          double out[10], cudaStream_t st);
-// Bvh4D::trace and interpolate_hit of caller rays (sr_trace_rays); error flags into counters[1].
+// Bvh4D::trace and interpolate_hit of caller rays (sr_trace_rays); error flags into counters[1], counters[2] zero at
+// the start; `rest`: n words of scratch.
 cudaError_t fast_trace_rays(const FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
-                            SrRayHit* hits, uint32_t* counters, cudaStream_t st);
+                            SrRayHit* hits, uint32_t* rest, uint32_t* counters, cudaStream_t st);
 // The device HDR image (level 0) of observer `i` of the last batch, for side outputs.
 float4* fast_batch_hdr(FastCtx& c, uint32_t pix_base_of_obs);
 
