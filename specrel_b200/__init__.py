@@ -560,7 +560,7 @@ class Engine:
         doubles, direction, t_min, t_max) on the device. Returns a structured array of SrRayHit."""
         r = np.atleast_2d(np.asarray(rays, np.float64))
         n = len(r)
-        if n and (r.ndim != 2 or r.shape[1] < 8):
+        if n and (r.ndim != 2 or r.shape[1] < 10):
             raise ValueError("rays: n x 10 values")
         arr = np.zeros(max(n, 1), np.dtype(_lib.Ray))
         if n:

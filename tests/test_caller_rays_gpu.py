@@ -95,3 +95,9 @@ def test_equal_lambda_hits(engine):
         h = _check(engine, TIES, _rays(6, 4000, 0.0, at=at))
         ids = h["id"][h["slot"] != 0xFFFFFFFF]
         assert (ids >= n).any() and (ids < n).any()
+
+
+@pytest.mark.parametrize("shape", [(3, 1), (2, 4), (2, 8), (2, 9), (2, 10, 1)])
+def test_rays_of_too_few_values_are_refused(engine, bodies, shape):
+    with pytest.raises(ValueError):
+        engine.trace_rays(IDX, np.zeros(shape))
