@@ -437,9 +437,12 @@ __global__ void k_copy_range(const Chunk* chunks, const LTask* tasks, const uint
 // Small subtrees: one block builds the subtree of one node depth first in shared memory, as the
 // serial build does. Nodes go to `out + 2 * start` with links relative to the subtree's root.
 // ---------------------------------------------------------------------------------------------
+// pending: the left turns from the topmost node of at most SMALL primitives down to this subtree. A subtree is refused
+// where one block over that node would hold more than STACK nodes waiting, whatever part of it is built elsewhere.
 struct STask {
-    uint32_t start, count;
+    uint32_t start, count, pending;
 };
+constexpr uint32_t STACK = 64;
 struct SResult {
     uint32_t nodes, depth, max_leaf, bad;
 };
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(256) k_small_build(const STask* tasks, const u
     __shared__ uint32_t bc[32];
     __shared__ float part[8][16];
     __shared__ int red[16];
-    __shared__ uint32_t fs[64], fc[64], fpatch[64], fdepth[64];  // DFS frames
+    __shared__ uint32_t fs[STACK], fc[STACK], fpatch[STACK], fdepth[STACK];  // DFS frames
     __shared__ int sp, node_count, cur_leaf, cur_axis, max_depth, max_leaf, bad;
     __shared__ float cur_pos;
     __shared__ uint32_t cur_s, cur_c, cur_patch, cur_depth, cur_mid;
@@ -617,7 +620,7 @@ __global__ void __launch_bounds__(256) k_small_build(const STask* tasks, const u
             if (cur_patch != 0xFFFFFFFFu) o[cur_patch].right_or_first = (uint32_t)idx;
             if ((int)cur_depth > max_depth) max_depth = (int)cur_depth;
             if (!leaf) {
-                if (sp + 2 > 64) {
+                if (sp + tk.pending + 2 > STACK) {
                     bad = 2;
                 } else {
                     // Right pushed first, so the left subtree is built first; its node patches the
@@ -647,7 +650,7 @@ struct TinyShared {
     uint32_t bc[32];
     int red[16];
     uint32_t lefts[TINY / 32];  // the elements of the node that go left, a bit each
-    uint32_t fs[64], fc[64], fpatch[64], fdepth[64];
+    uint32_t fs[STACK], fc[STACK], fpatch[STACK], fdepth[STACK];
     uint32_t cur_s, cur_c, cur_patch, cur_depth;
     int sp, node_count, max_depth, max_leaf, bad;
 };
@@ -816,7 +819,7 @@ __global__ void __launch_bounds__(32 * WARPS_TINY) k_small_build_warp(const STas
             if (w.cur_patch != 0xFFFFFFFFu) o[w.cur_patch].right_or_first = (uint32_t)idx;
             if ((int)w.cur_depth > w.max_depth) w.max_depth = (int)w.cur_depth;
             if (!leaf) {
-                if (w.sp + 2 > 64) {
+                if (w.sp + tk.pending + 2 > STACK) {
                     w.bad = 2;
                 } else {
                     w.fs[w.sp] = s + mid; w.fc[w.sp] = c - mid; w.fpatch[w.sp] = (uint32_t)idx; w.fdepth[w.sp] = w.cur_depth + 1; ++w.sp;
@@ -933,13 +936,16 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
     struct HNode {
         float lo[4], hi[4];
         uint32_t start, count, seg;
+        uint32_t pending = 0;  // STask::pending
         int left = -1, right = -1, small = -1, leaf = 0;
     };
     // A subtree is handed to one block or warp from SMALL primitives down, from TINY when there are many:
     // one block takes 2048 primitives node by node, 2.2 us each, which is the whole build's chain (3.2 of
     // 5.1 ms for 12,672 primitives, 14.5 of 27 ms for 2M), where three more levels of the passes over all large
     // nodes cost 0.4 ms and leave subtrees that thousands of warps build at once. A few chunks of a scene
-    // cache's snapshot are below the line and take the block.
+    // cache's snapshot are below the line and take the block. Where splits peel a few off at a time each takes a
+    // level (110 us): 8,900 primitives of which 900 need 29 more levels 4.9 ms against 3.7; leaving nodes that keep
+    // 7/8 of their parent's four times to a block gave 4.7 there and took 1.5 times as long on other such chains.
     const uint32_t small_max = n > MANY ? TINY : SMALL;
     std::vector<HNode> hn;
     std::vector<STask> small;
@@ -959,7 +965,7 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
             any_large = true;
         } else {
             r.small = (int)small.size();
-            small.push_back({r.start, r.count});
+            small.push_back({r.start, r.count, 0u});
             small_owner.push_back((int)hn.size());
         }
         hn.push_back(r);
@@ -1047,7 +1053,8 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
                 ti.max_leaf = std::max(ti.max_leaf, hn[id].count);
                 continue;
             }
-            if (h.m == 0 || h.m == hn[id].count) {
+            const bool below = hn[id].count <= SMALL;
+            if (h.m == 0 || h.m == hn[id].count || (below && hn[id].pending + 2 > STACK)) {
                 info->unsupported = 1;
                 return cudaSuccess;
             }
@@ -1058,12 +1065,13 @@ cudaError_t gpu_bvh_build_forest(const float4* box, uint32_t n, const GpuSegment
                 ch.start = parts[side][0];
                 ch.count = parts[side][1];
                 ch.seg = hn[id].seg;
+                if (below) ch.pending = hn[id].pending + (side == 0 ? 1u : 0u);
                 const int cid = (int)hn.size();
                 if (ch.count > small_max) {
                     next.push_back((uint32_t)cid);
                 } else {
                     ch.small = (int)small.size();
-                    small.push_back({ch.start, ch.count});
+                    small.push_back({ch.start, ch.count, ch.pending});
                     small_owner.push_back(cid);
                 }
                 hn.push_back(ch);
