@@ -159,10 +159,17 @@ __global__ void __launch_bounds__(128) k_fan_fill(const SrGpuNode* nodes, uint32
     ref[(size_t)w * 32u + lane] = r;
 }
 
+static size_t fan_scratch(uint32_t n) { return 6 * (size_t)n * 4 + sizeof(FanCounts); }
+
 // Builds the layout (s.fan_*); s.fan_levels stays 0 where there is none: memory short, a tree that needs more than
-// FAN_LEVELS levels, or boxes that are not nested. `scratch`: 6 n + 1024 words.
-static cudaError_t fan_build(FastScene& s, const SrGpuNode* nodes, uint32_t n, uint32_t* scratch, cudaStream_t st) {
+// FAN_LEVELS levels, or boxes that are not nested.
+static cudaError_t fan_build(FastScene& s, const SrGpuNode* nodes, uint32_t n, cudaStream_t st) {
     s.fan_levels = 0;
+    if (s.scratch.ensure_grow(fan_scratch(n)) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaStreamSynchronize(st);
+    }
+    uint32_t* scratch = s.scratch.as<uint32_t>();
     uint32_t *parent = scratch, *acc = parent + n, *total = acc + n, *uref = total + n, *units = uref + n, *roots = units + n;
     FanCounts* fc = reinterpret_cast<FanCounts*>(roots + n);
     const uint32_t blocks = (n + 255) / 256;

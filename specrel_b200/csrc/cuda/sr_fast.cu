@@ -169,6 +169,21 @@ void fast_release(FastCtx& c) {
     c.graphs.clear();
 }
 
+// Launches whose rays walk alone (k_trace_lean) all the same: few of them through a small scene, where no
+// walk is long and the packet's two launches, bounds and queue cost more than they save. Trace time, lone
+// against packet: 37k tetrahedra, 320x200: 13 against 30 us, 16 frames of about that size 110 against 231, 8 of
+// 640x400 142 against 242, but 1920x1200 88 against 65; 111k, 320x200: 18 against 34, 8 of 640x400 194 against
+// 305; 147k, 640x400: 69 against 61, four of them 267 against 211.
+constexpr uint64_t LONE_PRIMS = 1u << 17;
+static bool lone_rays(uint64_t prims, uint64_t pixels) { return prims <= LONE_PRIMS && prims * pixels < 1ull << 36; }
+
+// The fan layout of a scene that has been waiting for it.
+static cudaError_t fan_ready(FastScene& s, const SceneDev& sd, cudaStream_t st) {
+    if (!s.fan_pending) return cudaSuccess;
+    s.fan_pending = false;
+    return fan_build(s, sd.nodes, sd.num_nodes, st);
+}
+
 cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_t n, uint32_t depth, uint32_t num_prims,
                        uint32_t max_leaf, cudaStream_t st) {
     // Captured batch graphs hold the scene's parameters (root box, octant stride, counts) and are
@@ -179,6 +194,7 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
     fast_release(c);
     s.num_wide = 0;
     s.fan_levels = 0;
+    s.fan_pending = false;
     s.depth = depth;
     s.empty = n == 0;
     s.max_leaf = max_leaf;
@@ -200,8 +216,11 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
     s.root_ref = 0;  // internal root: wide node 0 (the top levels come first)
     size_t temp = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, temp, (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, st);
-    const size_t fan_scratch = 6 * (size_t)n * 4 + sizeof(FanCounts);
-    if ((e = s.scratch.ensure(std::max(3 * (size_t)n * 4 + 64 + temp + 512, fan_scratch))) != cudaSuccess) return e;
+    const size_t own = 3 * (size_t)n * 4 + 64 + temp + 512;
+    if ((e = s.scratch.ensure(num_prims > LONE_PRIMS ? std::max(own, fan_scratch(n)) : own)) != cudaSuccess) {
+        cudaGetLastError();  // without room for the fan layout's, no fan layout
+        if ((e = s.scratch.ensure(own)) != cudaSuccess) return e;
+    }
     uint32_t* flags = s.scratch.as<uint32_t>();
     uint32_t* wid = flags + n;
     uint32_t* topid = wid + n;
@@ -241,7 +260,13 @@ cudaError_t fast_build(FastCtx& c, FastScene& s, const SrGpuNode* nodes, uint32_
                                                  s.copies, s.refs.as<uint2>(), s.up.as<uint32_t>(),
                                                  s.leafpar.as<uint32_t>());
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return fan_build(s, nodes, n, s.scratch.as<uint32_t>(), st);
+    // Most frames of a small scene walk alone, and it may be changed for every one of them (a dirty-range update of
+    // 12,672 tetrahedra took 397 us with this layout and 324 without): it is made when something wants it.
+    if (num_prims <= LONE_PRIMS) {
+        s.fan_pending = true;
+        return cudaStreamSynchronize(st);
+    }
+    return fan_build(s, nodes, n, st);
 }
 
 SrTuning fast_default_tuning(const FastCtx& c) {
@@ -881,13 +906,6 @@ struct FanTasks {
     uint32_t waste;     // FAN_WASTE or FAN_WASTE_SMALL
     uint32_t helpers;   // the first blocks, whose warps wait for the queue's entries
 };
-
-// Launches whose rays walk alone (k_trace_lean) all the same: few of them through a small scene, where no
-// walk is long and the packet's two launches, bounds and queue cost more than they save. Trace time, lone
-// against packet: 37k tetrahedra, 320x200: 13 against 30 us, 16 frames of about that size 110 against 231, 8 of
-// 640x400 142 against 242, but 1920x1200 88 against 65; 111k, 320x200: 18 against 34, 8 of 640x400 194 against
-// 305; 147k, 640x400: 69 against 61, four of them 267 against 211.
-static bool lone_rays(uint64_t prims, uint64_t pixels) { return prims <= 1u << 17 && prims * pixels < 1ull << 36; }
 
 // log2 of a tile's pixels: 64, or 8 where that leaves less than a tile per warp. Three engines' frames in turn, in
 // tiles of 8, 16 and 64: 16 accelerated bodies at 120x78 102, 138 and 151 us a frame, at 320x200 130, 152 and
@@ -1630,16 +1648,20 @@ __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const 
 // 3105; a million: 12.7 and 13.5 ms, 29.5 and 30.8 (11.7 and 19.3), 11.2 and 14.9.
 constexpr uint32_t RAYS_LONG = 1u << 16;
 
-cudaError_t fast_trace_rays(const FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
+cudaError_t fast_trace_rays(FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
                             SrRayHit* hits, uint32_t* rest, uint32_t* counters, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const WideScene ws = wide_scene(s, sd);
     const double *a = anchor;
     const uint32_t blocks = (n + 3) / 4;
+    if (s.usable && n <= RAYS_LONG) {
+        cudaError_t e = fan_ready(s, sd, st);
+        if (e != cudaSuccess) return e;
+    }
     if (!s.usable || s.fan_levels == 0 || n > RAYS_LONG) {
         k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, nullptr, hits, counters);
         return cudaGetLastError();
     }
+    const WideScene ws = wide_scene(s, sd);
     if (ws.oct_copies)
         k_trace_rays_fan<true><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
     else
@@ -1650,7 +1672,7 @@ cudaError_t fast_trace_rays(const FastScene& s, const SceneDev& sd, const double
 
 float4* fast_batch_hdr(FastCtx& c, uint32_t pyr_base) { return c.hdr.as<float4>() + pyr_base; }
 
-cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd,
+cudaError_t fast_render_batch(FastCtx& c, FastScene& s, const SrTuning& t, const SceneDev& sd,
                               const double anchor[4], const BBConst& bb, uint32_t* counters, const BatchRequest& r,
                               cudaStream_t st) {
     if (r.n == 0) return cudaSuccess;
@@ -1662,7 +1684,12 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     // The packet walk; counting runs take the per-lane order, whose work counts are the reference's.
     uint64_t pixels = 0;
     for (uint32_t i = 0; i < r.n; ++i) pixels += (uint64_t)r.u[i].size[0] * r.u[i].size[1];
-    bool packet = t.packet != 0 && !r.count_work && (s.empty || s.fan_levels != 0) && !lone_rays(sd.num_prims, pixels);
+    cudaError_t e;
+    bool packet = t.packet != 0 && !r.count_work && !lone_rays(sd.num_prims, pixels);
+    if (packet && !s.empty) {
+        if ((e = fan_ready(s, sd, st)) != cudaSuccess) return e;
+        packet = s.fan_levels != 0;
+    }
     Shape sh;
     uint32_t tile_w = t.tile_w, tile_h = t.tile_h;
     if (packet) {
@@ -1691,7 +1718,6 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
     }
     const uint32_t n = r.n, stride = n + 1;
     if ((uint64_t)sh.total_tiles * 32 >= (1ull << 32)) return cudaErrorInvalidValue;
-    cudaError_t e;
     // Buffers (grown on demand; a growth invalidates every captured graph).
     size_t old_hits = c.hits.bytes, old_hdr = c.hdr.bytes, old_U = c.inputs.bytes, old_sh = c.shadow.bytes, old_rgb = c.rgb.bytes;
     // The batch's inputs are one block, copied at once: uniforms, cameras, observers, prefix rows.
@@ -2029,7 +2055,7 @@ static bool readable_here(const void* p, size_t bytes) {
            bytes <= size - (at - base);
 }
 
-cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd, const double anchor[4],
+cudaError_t fast_adjoint(FastCtx& c, FastScene& s, const SrTuning& t, const SceneDev& sd, const double anchor[4],
                          const BBConst& bb, uint32_t* counters, const SrGpuUniforms& u, const SrCameraF64& cam,
                          const float* target, uint32_t level, bool frozen, uint32_t row0, uint32_t row1,
                          double out[10], cudaStream_t st) {

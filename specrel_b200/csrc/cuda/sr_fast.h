@@ -64,8 +64,10 @@ struct FastScene {
     DevMem boxes, refs, scratch;
     // Up links for the packet traversal's ordering of equal-lambda hits (WideScene::up / leafpar).
     DevMem up, leafpar;
-    // The packet walk's layout (sr_fan.cuh); fan_levels 0: none, the rays walk alone.
+    // The packet walk's layout (sr_fan.cuh); fan_levels 0: none, the rays walk alone. fan_pending: it is made when a
+    // frame or a list of rays first wants it (small scenes).
     DevMem fan_box, fan_ref;
+    bool fan_pending = false;
     uint32_t fan_root = 0, fan_levels = 0, num_fans = 0;
     uint32_t num_wide = 0;
     uint32_t depth = 0;
@@ -157,7 +159,7 @@ struct BatchRequest {
     bool no_image;                // only the HDR image is wanted: no bloom, no packed pixels
     cudaEvent_t* ev;              // optional: 5 events, after camera, trace, shading, stars, bloom
 };
-cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd,
+cudaError_t fast_render_batch(FastCtx& c, FastScene& s, const SrTuning& t, const SceneDev& sd,
                               const double anchor[4], const BBConst& bb, uint32_t* counters, const BatchRequest& r,
                               cudaStream_t st);
 // The gradient of sum((P_level(HDR) - P_level(target))^2) with respect to (rapidity, event) of one
@@ -167,13 +169,13 @@ cudaError_t fast_render_batch(FastCtx& c, const FastScene& s, const SrTuning& t,
 // outcomes (no forward frame; the finite-difference check of the gradient). Only rows
 // [row0, row1) of the loss level count (and the frame's pixel rows under them): the results of a
 // partition of the rows sum to the whole frame's.
-cudaError_t fast_adjoint(FastCtx& c, const FastScene& s, const SrTuning& t, const SceneDev& sd, const double anchor[4],
+cudaError_t fast_adjoint(FastCtx& c, FastScene& s, const SrTuning& t, const SceneDev& sd, const double anchor[4],
                          const BBConst& bb, uint32_t* counters, const SrGpuUniforms& u, const SrCameraF64& cam,
                          const float* target, uint32_t level, bool frozen, uint32_t row0, uint32_t row1,
                          double out[10], cudaStream_t st);
 // Bvh4D::trace and interpolate_hit of caller rays (sr_trace_rays); error flags into counters[1], counters[2] zero at
 // the start; `rest`: n words of scratch.
-cudaError_t fast_trace_rays(const FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
+cudaError_t fast_trace_rays(FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
                             SrRayHit* hits, uint32_t* rest, uint32_t* counters, cudaStream_t st);
 // The device HDR image (level 0) of observer `i` of the last batch, for side outputs.
 float4* fast_batch_hdr(FastCtx& c, uint32_t pix_base_of_obs);

@@ -112,3 +112,35 @@ def test_records_with_nans_and_infinities(engine, row, value):
         hits += int(hit.sum())
         broken += int((hit & (plain.hit_id % 7 == 0)).sum())
     assert broken > hits / 10  # they are met often
+
+
+@pytest.mark.parametrize("steps", ["frame", "rays", "lone frame", "lone rays frame", "layout frame", "rays layout rays frame",
+                                   "update lone frame rays", "rays update update rays frame"])
+def test_small_scenes_get_the_layout_when_wanted(engine, steps):
+    """A scene of at most 2^17 records has its fan layout made by the first large frame or list of rays after each
+    change: every order of changes and uses gives the plain path's frames and the same rays' hits."""
+    s = sr.synth_scene(1, 1, n_bodies=16)
+    p = s.packed()
+    engine.build_tubes(IDX, s)
+    rays = np.zeros((20000, 10))
+    d = np.random.default_rng(7).normal(size=(20000, 3))
+    rays[:, 0:4], rays[:, 4], rays[:, 5:8] = (-20.0, 5.0, 3.0, -4.0), -1.0, d / np.linalg.norm(d, axis=1, keepdims=True)
+    rays[:, 8], rays[:, 9] = 1e-3, 180.0
+    far = rays.copy()
+    far[:, 4:8], far[:, 8:10] = rays[:, 4:8].astype(np.float32) * np.float64(UP), rays[:, 8:10].astype(np.float32) / np.float64(UP)
+    for layout, step in enumerate(steps.split()):
+        if step == "update":
+            engine.update(IDX, s, node_ranges=[(0, len(p.nodes))], prim_ranges=[(0, len(p.geoms))])
+        elif step == "layout":
+            engine.set_layout(IDX, 1 + layout % 2)
+        elif step == "rays":
+            a, b = engine.trace_rays(IDX, rays), engine.trace_rays(IDX, far)
+            assert (a["slot"] == b["slot"]).all() and (a["slot"] != 0xFFFFFFFF).any()
+        else:
+            w, h = (1920, 1200) if step == "frame" else (320, 200)
+            u = sr.uniforms(sr.camera((-20.0, 5.0, 3.0, -4.0), 100.0, rapidity=(0.4, 0.1, -0.3)), w, h, 0, 1, 0,
+                            num_nodes=s.num_nodes, light_pos=s.light_pos)
+            fast, plain = (engine.render(IDX, u, path=path, aux=True) for path in (sr.SR_PATH_FAST, sr.SR_PATH_PLAIN))
+            _same(fast, plain)
+            assert (plain.hit_id != 0xFFFFFFFF).any()
+    engine.set_layout(IDX, 0)
