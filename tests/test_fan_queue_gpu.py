@@ -103,3 +103,33 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_nothing_behind(world):
     eng.synchronize()
     for u, cam in views:
         _exact(eng, u, cam)
+
+
+def test_engines_in_turn(world):
+    """Three engines' packet frames and batches queued one after the other without a wait between them: each engine's
+    launches may run beside another's, whose waiting warps must not keep them from their work."""
+    _, scene = world
+    engines = [sr.Engine(0) for _ in range(3)]
+    try:
+        views = [[_view(scene, w, h, rapidity=r) for w, h in ((640, 400), (95, 41), (320, 200))]
+                 for r in ((1.6, -1.4, 1.2), (-0.9, 0.8, 1.0), (0.3, -0.2, 0.4))]
+        n = sum(u.size[0] * u.size[1] for u, _ in views[0])
+        outs = [[torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(8)] for _ in engines]
+        for e in engines:
+            e.build_tubes(0, scene)
+        for turn in range(8):
+            for e, v, o in zip(engines, views, outs):
+                e.render_batch(0, [u for u, _ in v], o[turn].data_ptr(), n, cams=[c for _, c in v])
+                e.render_into(0, v[1][0], o[turn].data_ptr() + 4 * 640 * 400, cam=v[1][1])
+        for e, v, o in zip(engines, views, outs):
+            e.synchronize()
+            t = e.tuning(0)
+            t.packet = 0
+            e.set_tuning(0, t)
+            ref = np.zeros(n, np.uint32)
+            e.render_batch(0, [u for u, _ in v], ref.ctypes.data, n, cams=[c for _, c in v], device_output=False)
+            for x in o:
+                assert (x.cpu().numpy().view(np.uint32) == ref).all()
+    finally:
+        for e in engines:
+            e.close()
