@@ -388,12 +388,13 @@ def config5_measure(args, local, stream, eng, idx):
 
 
 def coherent_roof(sr, eng, scene, ptr, B, seed, work, trace_ms):
-    """The trace kernel's ceiling on this GPU, measured in this run: batches in which every pixel of
-    a frame traces that frame's centre ray (half_wh = 0), so the 32 lanes of a warp take the same
-    nodes and tests in step, no lane idles, and every load after a warp's first is an L1 hit. The
-    kernel's time on such batches, least squares (non-negative) over per-launch, per-node-visit,
-    per-tetrahedron-test and per-shadow-ray costs, gives the time the same kernel would take on the
-    real batch's work if its rays were coherent: the roof. frac = roof time / measured time.
+    """The trace kernels' ceiling on this GPU, measured in this run: batches in which every pixel of
+    a frame traces that frame's centre ray (half_wh = 0), so a tile's packet walks what one ray
+    would and its bounds hold nothing else. The launches' time on such batches, least squares
+    (non-negative) over per-launch, per-node-visit, per-tetrahedron-test and per-shadow-ray costs
+    (the work counted by the per-ray order, which the packet walk does not do), gives the time they
+    would take on the real batch's work if its rays were coherent: the roof. frac = roof time /
+    measured time, what the spread of a tile's rays costs.
     Centre rays vary by observer rapidity, yaw and pitch, slice (past cone, God's-eye, future
     cone) and shadows on / off, so the work mix varies across the fitted batches.
     Only for scenes without stars (the binned-star set-up divides by the pixel pitch)."""
@@ -433,9 +434,9 @@ def coherent_roof(sr, eng, scene, ptr, B, seed, work, trace_ms):
     return {
         "achieved": rays / (trace_ms / 1e3) / 1e6, "peak": rays / (roof_ms / 1e3) / 1e6, "unit": "Mrays/s",
         "frac": roof_ms / trace_ms, "roof_ms_per_launch": roof_ms,
-        "peak_kind": "measured in this run: the same kernel on warp-coherent batches (every pixel of a frame on "
-                     "its centre ray), its per-launch, per-node-visit, per-test and per-shadow-ray costs fitted "
-                     "and applied to this batch's counted work",
+        "peak_kind": "measured in this run: the same launches on coherent batches (every pixel of a frame on "
+                     "its centre ray), their per-launch, per-node-visit, per-test and per-shadow-ray costs (work "
+                     "as the per-ray order counts it) fitted and applied to this batch's counted work",
         "coherent_fit": {"batches": int(len(y)), "ms_per_launch": float(coef[0]),
                          "ns_per_node_visit": float(coef[1] * 1e6), "ns_per_tet_test": float(coef[2] * 1e6),
                          "ns_per_shadow_ray": float(coef[3] * 1e6),
@@ -610,10 +611,10 @@ def run_engine(args, rank, world, local):
             fresh_ms = max_over_ranks(sum(a.elapsed_time(b) for a, b in evs) / args.steps)
             del flush
 
-        # The dominant kernel (k_trace_lean: primary rays and the main light's shadow rays of all
-        # B observers in one launch), timed with CUDA events the library records on the launching
-        # stream around each phase of the same batch, then the traversal work of that batch
-        # (counting variant).
+        # The dominant kernels (k_fan_trace and k_fan_shadow: the primary rays of all B observers,
+        # then the main light's shadow rays), timed with CUDA events the library records on the
+        # launching stream around each phase of the same batch, then the traversal work of that
+        # batch as the per-ray order does it (counting variant).
         trace_ms, frame_ms, shade_ms, bloom_ms = [], [], [], []
         for _ in range(args.steps):
             t = eng.render_batch(0, us, ptr, B * RAYS_PER_FRAME, cams=c64, device_output=True, phases=True)
@@ -648,11 +649,9 @@ def run_engine(args, rank, world, local):
     value = total_rays / (ms_max / 1e3) / 1e6
     plain_value = total_rays / (plain_ms / 1e3) / 1e6
     e2e_value = total_rays / (e2e_ms / 1e3) / 1e6
-    # Algorithmic bytes of one launch of the trace kernel (B frames) in the B200 layout: one 72-byte
-    # wide node (two child boxes + references) per internal visit, one 80-byte hot record per
-    # tetrahedron test, for primary and shadow rays (the visits are the reference traversal's own),
-    # plus the 21 bytes of hit record, slot and shadow state written per ray.
-    trace_bytes = 72.0 * (work[0] + work[3]) + 80.0 * (work[2] + work[5]) + 21.0 * RAYS_PER_FRAME * B
+    # What the trace of B frames cannot do without: the 21 bytes of hit record, slot and shadow state
+    # written per ray, and the 80-byte hot record it ends on read once (at most one per ray).
+    trace_bytes = (21.0 + 80.0) * RAYS_PER_FRAME * B
     trace_s = float(np.median(trace_ms)) / 1e3
     achieved = trace_bytes / trace_s / 1e9
     peak, peak_kind = load_peaks()
@@ -673,26 +672,25 @@ def run_engine(args, rank, world, local):
                   "speedup_batched_over_plain": value / plain_value},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": (768 + 80) * B,
                 "d2h_bytes_per_step": 4 * RAYS_PER_FRAME * B},
-        # Kernels per step: camera, trace, shade, 6 bloom down, 5 bloom up, composite.
-        "gpu_launches": int(args.steps * 15),
-        # The trace kernel is not bound by HBM: its working set (the light cone's share of the
-        # tree) is served from L1 and L2, so the byte model below (every node visit and test
-        # counted as if fetched) exceeds the HBM roof. What binds it is instruction issue and L1
-        # latency (ncu summaries in profiles/); its roof is the same kernel's speed on
-        # warp-coherent rays, measured in this run (coherent_roof).
-        "roofline": {"bound": "issue", "kernel": "k_trace_lean",
+        # Kernels per step: camera, closest hits, shadow rays, shade, 4 bloom down, the coarse levels,
+        # 4 bloom up, composite.
+        "gpu_launches": int(args.steps * 14),
+        # The trace is not bound by HBM: its working set (the light cone's share of the tree) is
+        # served from L1 and L2, and the bytes it cannot do without are a few percent of the HBM
+        # roof. What binds it is instruction issue and fixed latencies (ncu summaries in
+        # profiles/); its roof is the same launches' speed on coherent rays, measured in this run
+        # (coherent_roof).
+        "roofline": {"bound": "issue", "kernel": "k_fan_trace, k_fan_shadow",
                      **(roof if roof is not None else
                         {"achieved": None, "peak": None, "unit": "Mrays/s", "frac": None,
                          "peak_kind": "not measured (--no-roof, or a scene with stars)"}),
                      "hbm_achieved_gbs": achieved, "hbm_peak_gbs": peak, "hbm_frac": achieved / peak,
                      "hbm_peak_kind": peak_kind,
-                     "note": "frac = the trace kernel's time on this batch's counted work at warp-coherent speed "
-                             "(fitted on coherent batches in this run) / its measured time: what divergence and "
-                             "cache misses cost. hbm_achieved_gbs = algorithmic bytes (72 B per node visit, 80 B "
-                             "per tetrahedron test, 21 B written per ray) / trace-kernel time; these bytes are "
-                             "mostly served by L1/L2, so hbm_frac > 1 says the kernel is not HBM-bound. DRAM "
-                             "traffic and warp-instruction counts come from ncu captures (profiles/), not from "
-                             "this run.",
+                     "note": "frac = the trace's time on this batch's counted work at coherent speed (fitted on "
+                             "coherent batches in this run) / its measured time. hbm_achieved_gbs = the bytes it "
+                             "cannot do without (21 B written and at most one 80 B record read per ray) / its "
+                             "time. per_frame_work is the per-ray order's. DRAM traffic and warp-instruction "
+                             "counts come from ncu captures (profiles/), not from this run.",
                      "traffic": None,
                      "algorithmic_bytes_per_launch": trace_bytes, "frames_per_launch": B,
                      "trace_ms_per_launch": trace_s * 1e3,
