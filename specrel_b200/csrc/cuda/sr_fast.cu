@@ -1562,10 +1562,10 @@ __global__ void __launch_bounds__(64) k_trace_rays(const SceneDev s, double a0, 
 // smallest lambda; when the box's entry parameter as computed is not beyond it, every box on the way to
 // k is entered before any hit so far (boxes hold their children's), so the reference tests k, and no
 // nearer one. A hit before its box's entry is rounding against the build's padding; boxes are culled only
-// 0.1% beyond the closest hit, so that one is met rather than culled, and the ray is then left to the
-// reference's own walk, a thread per ray (k_trace_rays, with the rays that the layouts do not take: with the whole
-// warp here, a list of them took up to 3 times as long). Of hits at equal lambda the reference keeps the one its
-// order meets first (packet_precedes).
+// 0.1% beyond the closest hit, so that one is met rather than culled, and the ray then takes the reference's own
+// walk, as the rays that the layouts do not take: here, the whole warp doing the same, or, with `rest`, listed for a
+// thread each (k_trace_rays). Of hits at equal lambda the reference keeps the one its order meets first
+// (packet_precedes).
 template <bool OCT>
 __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const __grid_constant__ WideScene ws, double a0, double a1,
                                                         double a2, double a3, const SrRay* rays, uint32_t n, uint32_t* rest,
@@ -1636,9 +1636,12 @@ __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const 
             st[depth++] = make_uint2(key, ref);
         }
     }
-    if (lane != 0) return;
-    if (reference) rest[atomicAdd(counters + 2, 1u)] = i;
-    else write_ray_hit(s, a0, a1, a2, a3, o, d, slot, best, hits + i);
+    if (reference && rest) {
+        if (lane == 0) rest[atomicAdd(counters + 2, 1u)] = i;
+        return;
+    }
+    if (reference) slot = trace_ref(s, o, d, r.t_min, r.t_max, &best, counters + 1);  // the same for every lane
+    if (lane == 0) write_ray_hit(s, a0, a1, a2, a3, o, d, slot, best, hits + i);
 }
 
 // Lists longer than this walk a ray per thread: a warp per ray shortens the longest ray's chain of loads, which a
@@ -1647,6 +1650,11 @@ __global__ void __launch_bounds__(128) k_trace_rays_fan(const SceneDev s, const 
 // 1842 and 1192), into 147k tetrahedra 867 and 844; 262,144: 2766 and 2700, 7193 and 7129 (3261 and 4310), 2297 and
 // 3105; a million: 12.7 and 13.5 ms, 29.5 and 30.8 (11.7 and 19.3), 11.2 and 14.9.
 constexpr uint32_t RAYS_LONG = 1u << 16;
+// Lists longer than this leave the rays that take the reference's walk to a second launch, a thread each; in a shorter
+// one their warps walk them at once, alone in it as they are: lists of nothing else, warps against threads, 4096 rays
+// into 8 accelerated bodies 616 and 845 us, into 64 of them 1039 and 2907; 16,384: 783 and 1031, 1816 and 2899; but
+// 65,536: 1188 and 1356, 4910 and 3432. The launch costs 2 us of a 69 us call.
+constexpr uint32_t RAYS_REST = 1u << 14;
 
 cudaError_t fast_trace_rays(FastScene& s, const SceneDev& sd, const double anchor[4], const SrRay* rays, uint32_t n,
                             SrRayHit* hits, uint32_t* rest, uint32_t* counters, cudaStream_t st) {
@@ -1662,11 +1670,12 @@ cudaError_t fast_trace_rays(FastScene& s, const SceneDev& sd, const double ancho
         return cudaGetLastError();
     }
     const WideScene ws = wide_scene(s, sd);
+    if (n <= RAYS_REST) rest = nullptr;
     if (ws.oct_copies)
         k_trace_rays_fan<true><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
     else
         k_trace_rays_fan<false><<<blocks, 128, 0, st>>>(sd, ws, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
-    k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
+    if (rest) k_trace_rays<<<(n + 63) / 64, 64, 0, st>>>(sd, a[0], a[1], a[2], a[3], rays, n, rest, hits, counters);
     return cudaGetLastError();
 }
 

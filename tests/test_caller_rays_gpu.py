@@ -70,10 +70,11 @@ def test_lists_on_both_sides_of_the_line(engine, bodies, n):
     assert part.tobytes() == h[n - 300:].tobytes()
 
 
-def test_rays_the_layout_does_not_take_among_others(engine, bodies):
+@pytest.mark.parametrize("n", [3000, 1 << 14, (1 << 14) + 1])  # walked by their warps, and listed
+def test_rays_the_layout_does_not_take_among_others(engine, bodies, n):
     """Negative and NaN ranges, endless ones and values beyond 1e12, scattered over a list: every ray has the hit it
     has alone, and the list's order does not matter."""
-    rays = _rays(5, 3000)
+    rays = _rays(5, n)
     odd = {0: (8, -1.0), 5: (8, np.nan), 11: (9, np.inf), 17: (9, 0.0), 23: (0, 1e13), 29: (9, np.nan), 31: (9, -1.0)}
     for k, (col, v) in odd.items():
         rays[k::97, col] = v
